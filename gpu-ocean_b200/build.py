@@ -25,7 +25,7 @@ LIB = os.path.join(HERE, "lib", "libgocean.so")
 DEBUG_LIB = os.path.join(HERE, "lib", "libgocean_debug.so")
 DEBUG_UNITS = ("batch.cu", "pair_batch_frame.cu", "pair_batch_int_f0.cu", "pair_batch_int_f1.cu",
                "pair_batch_int_f2.cu", "pair_single_frame.cu", "pair_single_int_f0.cu", "pair_single_int_f1.cu",
-               "pair_single_int_f2.cu", "stage_launch.cu")
+               "pair_single_int_f2.cu", "stage_launch.cu", "tile_launch.cu")
 INCLUDE = os.path.join(ROOT, "include")
 
 NVCC_FLAGS = [

@@ -1674,7 +1674,7 @@ int go_traj_step(go_domain* d, void* stream, float dt, float wind_stress_t, cons
     a1.qn_eta = q_n->eta; a1.qn_hu = q_n->hu; a1.qn_hv = q_n->hv; a1.pqn = q_n->pitch / 4;
     rc = go_launch_stage(d, s, a0);
     if (rc) return rc;
-    return go_launch_stage(d, s, a1);
+    return go_launch_stage(d, s, a1, true);
 }
 
 int go_obs_misfit(void* stream, const go_state* q, int nx, int ny, int n_obs, const int* obs_ij,

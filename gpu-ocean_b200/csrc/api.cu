@@ -108,6 +108,8 @@ StageArgs go_stage_args(const go_domain* d, float dt, int rk_step, const float* 
     a.debug = d->debug;
     a.neg_zero = -0.0f;
     a.fric = go_friction_mode(d);
+    a.deep_lo = deep_depth(a.k);
+    a.deep_hi = deep_end(a.k);
     return a;
 }
 
@@ -242,6 +244,7 @@ int go_domain_create(const go_domain_desc* desc, go_domain** out) {
     d->rows_per_block = go_auto_rows(s.nx, s.ny, d->shape);
     d->arith = GO_ARITH_RCP;
     d->has_land = 1;
+    d->auto_launch = 1;
     cudaError_t e = cudaGetDevice(&d->device);
     if (e == cudaSuccess) e = cudaMalloc(&d->d_frows, sizeof(float) * (s.ny + 4));
     if (e == cudaSuccess) e = cudaMemset(d->d_frows, 0, sizeof(float) * (s.ny + 4));
@@ -252,6 +255,11 @@ int go_domain_create(const go_domain_desc* desc, go_domain** out) {
         cudaFree(d->d_status);
         delete d;
         return go_fail(GO_ERR_CUDA, "domain allocation failed: %s", cudaGetErrorString(e));
+    }
+    const int rc = go_tile_setup(d);
+    if (rc) {
+        go_domain_destroy(d);
+        return rc;
     }
     *out = d;
     return GO_OK;
@@ -313,6 +321,7 @@ int go_domain_set_launch(go_domain* d, int shape, int rows_per_block) {
     if (rows_per_block < 1) return go_fail(GO_ERR_INVALID, "rows_per_block must be >= 1");
     d->shape = shape;
     d->rows_per_block = rows_per_block;
+    d->auto_launch = 0;
     return GO_OK;
 }
 
@@ -326,6 +335,7 @@ int go_domain_set_arith(go_domain* d, int mode) {
 int go_domain_set_land(go_domain* d, int may_have_land) {
     if (!d) return go_fail(GO_ERR_INVALID, "null domain");
     d->has_land = may_have_land ? 1 : 0;
+    d->land_told = d->has_land;
     return GO_OK;
 }
 
@@ -416,18 +426,20 @@ int go_cdklm_step(go_domain* d, void* stream, int n_steps, float dt, float wind_
     const StageArgs a1 = go_stage_args(d, dt, 1, eta1, hu1, hv1, pitch1 / 4, eta0, hu0, hv0, pitch0 / 4, Hi,
                                        Hi_pitch / 4, land_value, wind_stress_t);
     const bool open = go_has_open_bc(d);
+    if (!open && go_tile_stage(d, a0) && go_tile_stage(d, a1) && go_tile_steps_fit(d))
+        return go_launch_tile_steps(d, s, a0, n_steps);
     PreparedStage p0, p1;
     rc = go_prepare_stage(d, a0, &p0);
     if (!rc) rc = go_prepare_stage(d, a1, &p1);
     if (rc) return rc;
     for (int n = 0; n < n_steps; ++n) {
-        rc = go_launch_prepared(d, s, p0);
+        rc = go_launch_prepared(d, s, p0, n > 0 && !open);
         // open boundaries: the reference's ghost sequence after each stage
         // (CDKLM16.py:537-540, 585-586); the stage kernel's own periodic
         // images are redone in order after the open kinds of the other axis
         if (!rc && open) rc = go_boundary_condition(d, stream, eta1, hu1, hv1, pitch1);
         if (rc) return rc;
-        rc = go_launch_prepared(d, s, p1);
+        rc = go_launch_prepared(d, s, p1, !open);
         if (!rc && open) rc = go_boundary_condition(d, stream, eta0, hu0, hv0, pitch0);
         if (rc) return rc;
     }

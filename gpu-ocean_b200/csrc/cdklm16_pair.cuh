@@ -161,6 +161,37 @@ __device__ __forceinline__ void pflux(float2 hm, float2 um, float2 vm, float2 hp
     }
 }
 
+// x times a constant: a scalar (two scalar multiplies) or a pair (one packed).
+__device__ __forceinline__ float2 pmulc(float2 x, float c, float2) { return pscale(x, c); }
+__device__ __forceinline__ float2 pmulc(float2 x, float2 c, float2 nz) { return pmul_nz(x, c, nz); }
+
+// pflux in deep water (deep.cuh): two wet faces of an open fan, the general
+// form's arithmetic without its selections.
+template <class C>
+__device__ __forceinline__ void pflux_deep(float2 hm, float2 um, float2 vm, float2 hp, float2 up, float2 vp, C half_g,
+                                           C g, float2 nz, float2& F0, float2& F1, float2& F2) {
+    auto pmul = [&](float2 x, float2 y) { return pmul_nz(x, y, nz); };
+    const float2 Fp0 = pmul(hp, up), Fm0 = pmul(hm, um);
+    const float2 Fp1 = padd(pmul(Fp0, up), pmul(pmulc(hp, half_g, nz), hp));
+    const float2 Fm1 = padd(pmul(Fm0, um), pmul(pmulc(hm, half_g, nz), hm));
+    const float2 gp = pmulc(hp, g, nz), gm = pmulc(hm, g, nz);
+    const float2 cp = make_float2(sqrtf(gp.x), sqrtf(gp.y)), cm = make_float2(sqrtf(gm.x), sqrtf(gm.y));
+    const float2 a1 = psub(um, cm), a2 = psub(up, cp);
+    const float2 b1 = padd(um, cm), b2 = padd(up, cp);
+    const float2 am = make_float2(fmin3(a1.x, a2.x, 0.0f), fmin3(a1.y, a2.y, 0.0f));
+    const float2 ap = make_float2(fmax3(b1.x, b2.x, 0.0f), fmax3(b1.y, b2.y, 0.0f));
+    const float2 d = psub(ap, am);
+    const float2 apam = pmul(ap, am);
+    const float2 n0 = padd(psub(pmul(ap, Fm0), pmul(am, Fp0)), pmul(apam, psub(hp, hm)));
+    const float2 n1 = padd(psub(pmul(ap, Fm1), pmul(am, Fp1)), pmul(apam, psub(Fp0, Fm0)));
+    const float2 rd = make_float2(rcp_approx(d.x), rcp_approx(d.y));
+    F0 = pmul(n0, rd);
+    F1 = pmul(n1, rd);
+    // upwinded tangential flux: the product of the chosen side
+    const float2 s = padd(um, up);
+    F2 = pmul(psel(s.x > 0.0f, s.y > 0.0f, Fm0, Fp0), psel(s.x > 0.0f, s.y > 0.0f, vm, vp));
+}
+
 // Face states of two faces (one float2 lane each): minus side (hm, um, vm),
 // plus side (hp, up, vp); un normal, ut tangential.
 struct PFace {

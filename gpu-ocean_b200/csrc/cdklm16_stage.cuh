@@ -41,6 +41,7 @@
 
 #include "cdklm16_device.cuh"
 #include "checked.cuh"
+#include "deep.cuh"
 
 namespace go {
 
@@ -66,6 +67,7 @@ struct StageArgs {
     float neg_zero;              // -0.0f: the addend of the packed products (column-pair kernel)
     int fric;                    // friction law kFric* (column-pair kernel; the marching kernel has it as a template)
     unsigned debug;              // GO_DEBUG_* test hooks (go_domain_set_debug), 0 in normal runs
+    float deep_lo, deep_hi;      // corner depths of deep water lie in [deep_lo, deep_hi) (deep.cuh)
 };
 
 // Friction law selector.

@@ -35,6 +35,9 @@ struct go_domain {
     int own_side;            // go_domain_create's handles may create them (not the allocation-free step)
     int stage_launches;      // kernel launches the last RK stage issued
     unsigned debug;          // GO_DEBUG_* test hooks
+    int auto_launch;         // launch choice left to the library (until a shape is set)
+    int land_told;           // go_domain_set_land said that the bathymetry may hold land
+    int tile_steps_blocks;   // most tiles of a cooperative launch of many steps (0: none)
 };
 
 // Records the message of a failed call (go_last_error) and returns code.
@@ -74,8 +77,17 @@ namespace go { struct Variant; }
 // Kernel variant of a domain (stage_launch.cu).
 go::Variant go_variant(const go_domain* d);
 
-// One single-domain stage launch (stage_launch.cu).
-int go_launch_stage(go_domain* d, cudaStream_t s, const go::StageArgs& a);
+// One single-domain stage launch (stage_launch.cu).  follows: the launch before
+// it on the stream is a stage of the same domain in the same call.
+int go_launch_stage(go_domain* d, cudaStream_t s, const go::StageArgs& a, bool follows = false);
+
+// Tile stage kernel (tile_launch.cu): set-up of a domain that may run it,
+// whether a stage does, and its launches.
+int go_tile_setup(go_domain* d);
+bool go_tile_stage(const go_domain* d, const go::StageArgs& a);
+int go_launch_tile(go_domain* d, cudaStream_t s, const go::StageArgs& a, bool follows);
+bool go_tile_steps_fit(const go_domain* d);
+int go_launch_tile_steps(go_domain* d, cudaStream_t s, const go::StageArgs& a, int n);
 
 // Column-pair shape (pair_launch.cu).
 bool go_pair_shape(int shape);
@@ -87,4 +99,4 @@ int go_launch_pair(go_domain* d, cudaStream_t s, const go::StageArgs& a, const g
 // many times (stage_launch.cu).
 struct PreparedStage;
 int go_prepare_stage(go_domain* d, const go::StageArgs& a, PreparedStage* p);
-int go_launch_prepared(go_domain* d, cudaStream_t s, const PreparedStage& p);
+int go_launch_prepared(go_domain* d, cudaStream_t s, const PreparedStage& p, bool follows = false);

@@ -134,5 +134,5 @@ cudaError_t pair_launch_periodic_columns(const StageArgs* args, int n, int max_n
 struct PreparedStage {
     go::StageArgs a;
     go::PairMapParams mp;
-    bool pair, tma;
+    bool pair, tma, tile;
 };

@@ -1,5 +1,5 @@
-// Single-domain stage launches: the column-pair kernel (pair_launch.cu) or
-// a variant of the marching kernel.
+// Single-domain stage launches: the tile kernel (tile_launch.cu), the
+// column-pair kernel (pair_launch.cu) or a variant of the marching kernel.
 #include "pair_dispatch.cuh"
 
 using namespace go;
@@ -32,7 +32,8 @@ Variant go_variant(const go_domain* d) {
 
 int go_prepare_stage(go_domain* d, const StageArgs& a, PreparedStage* p) {
     p->a = a;
-    p->pair = go_pair_shape(d->shape);
+    p->tile = go_tile_stage(d, a);
+    p->pair = !p->tile && go_pair_shape(d->shape);
     p->tma = false;
     if (!p->pair) return GO_OK;
     if (d->own_side && !d->side) {
@@ -47,7 +48,8 @@ int go_prepare_stage(go_domain* d, const StageArgs& a, PreparedStage* p) {
     return go_prepare_pair(a, &p->mp, &p->tma);
 }
 
-int go_launch_prepared(go_domain* d, cudaStream_t s, const PreparedStage& p) {
+int go_launch_prepared(go_domain* d, cudaStream_t s, const PreparedStage& p, bool follows) {
+    if (p.tile) return go_launch_tile(d, s, p.a, follows);
     if (p.pair) return go_launch_pair(d, s, p.a, p.mp, p.tma);
     d->stage_launches = 1;
     SingleLaunch L{&p.a, s};
@@ -56,9 +58,9 @@ int go_launch_prepared(go_domain* d, cudaStream_t s, const PreparedStage& p) {
     return GO_OK;
 }
 
-int go_launch_stage(go_domain* d, cudaStream_t s, const StageArgs& a) {
+int go_launch_stage(go_domain* d, cudaStream_t s, const StageArgs& a, bool follows) {
     PreparedStage p;
     int rc = go_prepare_stage(d, a, &p);
-    if (!rc) rc = go_launch_prepared(d, s, p);
+    if (!rc) rc = go_launch_prepared(d, s, p, follows);
     return rc;
 }

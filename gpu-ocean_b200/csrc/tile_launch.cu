@@ -1,0 +1,86 @@
+// Launches of the tile stage kernels (cdklm16_tile.cuh).
+#include "pair_dispatch.cuh"
+
+#include "cdklm16_tile.cuh"
+
+using namespace go;
+
+namespace {
+
+constexpr long long kTileCells = 1150LL * 1000LL, kTileLandCells = 350LL * 1000LL;
+
+dim3 tile_grid(const Scheme& k) { return dim3((k.nx + kTileX - 1) / kTileX, (k.ny + kTileY - 1) / kTileY); }
+
+}  // namespace
+
+int go_tile_setup(go_domain* d) {
+    if ((long long)d->k.nx * d->k.ny >= kTileCells) return GO_OK;
+    const int bytes = (int)sizeof(TileSmem);
+    GO_CUDA(cudaFuncSetAttribute(cdklm_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    GO_CUDA(cudaFuncSetAttribute(cdklm_tile_steps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    int sms = 0, coop = 0;
+    GO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device));
+    GO_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, d->device));
+    d->tile_steps_blocks = coop ? sms : 0;
+    return GO_OK;
+}
+
+// Grids that run the tile kernel unless a launch shape was set.  Measured on a
+// B200, us per RK2 step, tile against the marching kernel's default; one
+// simulator, and three on their own streams: 512^2 17.2 / 28.8 and 11.7 / 18.9,
+// 768^2 30.7 / 46.3 and 23.8 / 29.5, 1024^2 48.8 / 67.1 and 44.6 / 46.4, 1280^2
+// 70.8 / 99.6 but 71.0 / 68.1.  With land (a seventh of the corners, in patches
+// of 20 cells, so that few tiles are deep): 512^2 23.7 / 33.0 and 18.4 / 23.6,
+// 640^2 34.4 / 39.3 but 26.5 / 24.6, 1024^2 68.9 / 78.1 but 63.9 / 52.5.
+bool go_tile_stage(const go_domain* d, const StageArgs& a) {
+    const long long cells = (long long)a.k.nx * a.k.ny;
+    // 32-bit byte offsets into every array
+    auto fits = [&](int pitch) { return (long long)(a.k.ny + 5) * pitch * 4 < (1LL << 32); };
+    return d->auto_launch && cells < (d->land_told ? kTileLandCells : kTileCells) && d->arith == GO_ARITH_RCP &&
+           !go_general_north(d) && fits(a.pin) && fits(a.pout) && fits(a.pqn) && fits(a.phi);
+}
+
+// One stage.  follows: the launch before it on the stream is a tile stage of
+// the same call, so this one is a programmatic dependent launch: its blocks
+// are scheduled, and read the corners, while that one's last blocks run.
+// Measured on a B200, us per RK2 step without / with: 64 x 48 12.4 / 9.2,
+// 512^2 20.6 / 16.7, 1024^2 53.4 / 48.5.
+int go_launch_tile(go_domain* d, cudaStream_t s, const StageArgs& a, bool follows) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = tile_grid(a.k);
+    cfg.blockDim = dim3(kTileThreads);
+    cfg.dynamicSmemBytes = sizeof(TileSmem);
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = follows ? 1 : 0;
+    d->stage_launches = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, cdklm_tile_kernel, a, tile_const(a.k));
+    if (e != cudaSuccess) return go_fail(GO_ERR_CUDA, "stage launch (tile) failed: %s", cudaGetErrorString(e));
+    return GO_OK;
+}
+
+// Grids of at most one tile per SM run all the steps of a call in one
+// cooperative launch.  Measured on a B200 for 10 steps, us per step and (three
+// simulators on their own streams) us per call, against one launch per stage:
+// 64 x 48 8.7 / 9.2 and 33 / 51; 256^2 10.0 / 10.6 and 57 / 59; 384^2 (288
+// tiles) 11.4 / 13.2 but 114 / 76, since launches of two tiles per SM leave the
+// simulators no room beside one another.
+bool go_tile_steps_fit(const go_domain* d) {
+    const dim3 g = tile_grid(d->k);
+    return (int)(g.x * g.y) <= d->tile_steps_blocks;
+}
+
+int go_launch_tile_steps(go_domain* d, cudaStream_t s, const StageArgs& a, int n) {
+    if (n < 1) return GO_OK;
+    StageArgs args = a;
+    TileConst tc = tile_const(a.k);
+    void* params[] = {&args, &tc, &n};
+    d->stage_launches = 1;
+    const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(cdklm_tile_steps_kernel),
+                                                      tile_grid(a.k), dim3(kTileThreads), params, sizeof(TileSmem), s);
+    if (e != cudaSuccess) return go_fail(GO_ERR_CUDA, "step launch (tiles) failed: %s", cudaGetErrorString(e));
+    return GO_OK;
+}
