@@ -3,6 +3,9 @@
 // Build: gpu-ocean_b200/build.py compiles every csrc/*.cu for sm_100a with
 // the reference's floating-point flags (CDKLM16.py:196-200):
 // --ftz=true --prec-div=false --prec-sqrt=false --fmad=false.
+#include <math.h>
+
+#include <algorithm>
 #include <string>
 
 #include "pair_dispatch.cuh"
@@ -29,6 +32,34 @@ int go_check_pitch(int pitch_bytes, int min_floats, const char* what) {
     return GO_OK;
 }
 
+// Rows per block strip of the column-pair kernel, in whole ring chunks of 3
+// rows.  A strip costs its rows and about 2 more for its priming; w waves of
+// strips take the whole waves in full, and of the last, partly filled one a
+// share that grows with its filling f (a lone strip runs in about 0.35 of the
+// time that it takes among a full wave), and less per row when several waves
+// overlap than when all strips run in step.  Beside other work on the chip the
+// waves do not show and the priming alone counts, which the last factor weighs
+// in.  The numbers are a fit to heights of 9 .. 120 rows on ten grids of 1280^2 ..
+// 4096^2 (B200, us per RK2 step, one simulator and three on their own streams;
+// the height taken / others): 1280^2 12 rows 87 and 61 / 18 97 and 60, 2048^2 30
+// rows 177 and 134 / 24 209 and 136, 3072^2 66 rows 350 and 285 / 36 373 and 289,
+// 4096^2 60 rows 597 and 513 / 24 585 and 528, 42 611 and 517.
+static int pair_rows(int nx, int ny) {
+    const long long slots = 148LL * go::shape_blocks_per_sm(GO_SHAPE_PAIR);
+    const int useful = go::shape_block_width(GO_SHAPE_PAIR) - 4;
+    const long long strips = (nx + useful - 1) / useful;
+    int best = 3;
+    double best_cost = -1.0;
+    for (int r = 3; r <= 120; r += 3) {
+        const double w = (double)(strips * ((std::max(ny - 4, 1) + r - 1) / r)) / (double)slots;
+        const double whole = floor(w), f = w - whole;
+        const double alone = (r + 2) * (whole + (f > 0.0 ? 0.35 + 0.65 * f : 0.0)) * (2.2 + 0.2 / ceil(w));
+        const double cost = alone * (1.0 + 1.5 / r);
+        if (best_cost < 0.0 || cost < best_cost) { best = r; best_cost = cost; }
+    }
+    return best;
+}
+
 // Rows per block strip.  A block's cost is about (rows + 4) row steps: it
 // recomputes the 4 rows above and below its strip before its first output
 // row.  The strip height r in {2, 4, 8, 16, 24} minimises
@@ -37,44 +68,50 @@ int go_check_pitch(int pitch_bytes, int min_floats, const char* what) {
 // strip on a tie.  Measured on a B200 (us per RK2 step, default shape):
 // 1024^2 picks 16 (66; 8 rows: 70), 4096^2 picks 24 (720; 16 rows: 727).
 int go_auto_rows(int nx, int ny, int shape) {
+    if (go_pair_shape(shape)) return pair_rows(nx, ny);
     const int useful = go::shape_block_width(shape) - 4;
     const long long strips = (nx + useful - 1) / useful;
     const long long slots = 148LL * go::shape_blocks_per_sm(shape);
     static const int kRows[] = {2, 4, 8, 16, 24};
-    // column-pair shapes: heights in whole ring chunks of 3 rows; priming a
-    // strip costs about 2 rows
-    static const int kPairRows[] = {3, 6, 12, 24, 36, 48, 72, 96};
-    const bool pair = go_pair_shape(shape);
-    const int* rows = pair ? kPairRows : kRows;
-    const int n = pair ? 8 : 5;
-    const int extra = pair ? 2 : 4;
-    int best = rows[0];
+    int best = kRows[0];
     long long best_cost = -1;
-    for (int i = 0; i < n; ++i) {
-        const int r = rows[i];
+    for (int r : kRows) {
         const long long blocks = strips * ((ny + r - 1) / r);
-        const long long cost = ((blocks + slots - 1) / slots) * (r + extra);
+        const long long cost = ((blocks + slots - 1) / slots) * (r + 4);
         if (best_cost < 0 || cost <= best_cost) { best = r; best_cost = cost; }
     }
     return best;
 }
 
-// Default launch shape: the column-pair kernel (shape 8) from about 1500^2
-// cells up (measured on a B200, us per step, shapes 4 / 5 / 8, walls N/S and
-// periodic E/W: 1536^2 126 / 128 / 118, 2048^2 208 / 203 / 200, 2560^2
-// 308 / 292 / 262, 3072^2 429 / 399 / 373, 4096^2 720 / 686 / 583; at
-// 1024^2 and below the pair kernel's separate boundary-frame launch does not
-// pay: 68 / 72 / 71 and 29 / 32 / 36 at 512^2).  Below that a read-ahead shape (5,
-// or 6 for widths that 96-wide blocks cover with less waste) once the grid
-// needs more than one wave of blocks, where the ring hides the load
-// latency; in a single wave the register prefetch of 128 x 5 blocks
+// A read-ahead shape (5, or 6 for widths that 96-wide blocks cover with less
+// waste) once the grid needs more than one wave of blocks, where the ring hides
+// the load latency; in a single wave the register prefetch of 128 x 5 blocks
 // (shape 4) is faster (1024^2 and below lose 6-9% with the ring).
-int go_auto_shape(int nx, int ny) {
-    if ((long long)nx * ny >= kPairAutoCells) return GO_SHAPE_PAIR;
+static int march_shape(int nx, int ny) {
     const int ring = go::ring_shape(go::shape_columns(5, nx), go::shape_columns(6, nx));
     const int rows = go_auto_rows(nx, ny, ring);
     const long long blocks = go::shape_columns(ring, nx) / go::shape_block_width(ring) * ((ny + rows - 1) / rows);
     return blocks > 148LL * go::shape_blocks_per_sm(ring) ? ring : 4;
+}
+
+// Default launch shape of the grids that the tile kernel leaves (go_tile_stage):
+// the column-pair kernel (shape 8) from about 1070^2 cells up.  Measured on a
+// B200, us per step, best of shapes 4 .. 6 / shape 8 (walls N/S, periodic E/W),
+// one simulator and three on their own streams: 1280^2 100 / 87 and 68 / 60,
+// 1501 x 1203 109 / 99 and 75 / 68, 2048^2 203 / 174 and 164 / 135, 4096^2
+// 684 / 584 and 641 / 528.
+int go_auto_shape(int nx, int ny) {
+    if ((long long)nx * ny >= kPairAutoCells) return GO_SHAPE_PAIR;
+    return march_shape(nx, ny);
+}
+
+// The same for bathymetry with land, whose branches cost the two-column warps of
+// the column-pair kernel more: the marching kernel up to 3500^2 cells (per-cell
+// wind, a seventh of the corners land in patches of 20 cells; best of shapes
+// 4 .. 6 / shape 8: 1536^2 149 / 166 and 112 / 160, 2048^2 228 / 268 and 188 / 220,
+// 3072^2 467 / 487 and 411 / 446, 4096^2 786 / 779 and 740 / 754).
+static int auto_shape_land(int nx, int ny) {
+    return (long long)nx * ny < 3500LL * 3500LL ? march_shape(nx, ny) : go_auto_shape(nx, ny);
 }
 
 int go_friction_mode(const go_domain* d) {
@@ -336,6 +373,10 @@ int go_domain_set_land(go_domain* d, int may_have_land) {
     if (!d) return go_fail(GO_ERR_INVALID, "null domain");
     d->has_land = may_have_land ? 1 : 0;
     d->land_told = d->has_land;
+    if (d->auto_launch) {
+        d->shape = d->land_told ? auto_shape_land(d->k.nx, d->k.ny) : go_auto_shape(d->k.nx, d->k.ny);
+        d->rows_per_block = go_auto_rows(d->k.nx, d->k.ny, d->shape);
+    }
     return GO_OK;
 }
 

@@ -25,7 +25,7 @@ constexpr int kPairUnroll = 1;
 constexpr int kPairFrameRows = 8;
 // default-shape thresholds: a grid of at least this many cells, a batch
 // whose members hold at least this many together
-constexpr long long kPairAutoCells = 1500LL * 1500LL;
+constexpr long long kPairAutoCells = 1150LL * 1000LL;
 constexpr long long kPairAutoBatchCells = 2LL << 20;
 
 // The block grid of an nx x ny domain (see PairGrid): the region of TMA
