@@ -3,12 +3,11 @@
 // Build: gpu-ocean_b200/build.py compiles every csrc/*.cu for sm_100a with
 // the reference's floating-point flags (CDKLM16.py:196-200):
 // --ftz=true --prec-div=false --prec-sqrt=false --fmad=false.
-#include <math.h>
-
 #include <algorithm>
 #include <string>
 
 #include "pair_dispatch.cuh"
+#include "pair_rows.h"
 #include "trace.h"
 
 using namespace go;
@@ -45,16 +44,11 @@ int go_check_pitch(int pitch_bytes, int min_floats, const char* what) {
 // rows 177 and 134 / 24 209 and 136, 3072^2 66 rows 350 and 285 / 36 373 and 289,
 // 4096^2 60 rows 597 and 513 / 24 585 and 528, 42 611 and 517.
 static int pair_rows(int nx, int ny) {
-    const long long slots = 148LL * go::shape_blocks_per_sm(GO_SHAPE_PAIR);
-    const int useful = go::shape_block_width(GO_SHAPE_PAIR) - 4;
-    const long long strips = (nx + useful - 1) / useful;
+    const long long strips = go::shape_columns(GO_SHAPE_PAIR, nx) / go::shape_block_width(GO_SHAPE_PAIR);
     int best = 3;
     double best_cost = -1.0;
     for (int r = 3; r <= 120; r += 3) {
-        const double w = (double)(strips * ((std::max(ny - 4, 1) + r - 1) / r)) / (double)slots;
-        const double whole = floor(w), f = w - whole;
-        const double alone = (r + 2) * (whole + (f > 0.0 ? 0.35 + 0.65 * f : 0.0)) * (2.2 + 0.2 / ceil(w));
-        const double cost = alone * (1.0 + 1.5 / r);
+        const double cost = go::pair_strip_cost(strips * ((std::max(ny - 4, 1) + r - 1) / r), r) * (1.0 + 1.5 / r);
         if (best_cost < 0.0 || cost < best_cost) { best = r; best_cost = cost; }
     }
     return best;

@@ -12,6 +12,8 @@
 #include "grf.cuh"
 #include "trace.h"
 #include "pair_dispatch.cuh"
+#include "pair_rows.h"
+#include "tile_batch.h"
 
 using namespace go;
 
@@ -62,6 +64,10 @@ struct go_batch {
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int shape = 4, rows = 32, blocks = 0;
+    // tile kernel: the default launch (until go_batch_set_launch) of members
+    // it suits (batch_tile)
+    bool auto_launch = true, tile = false;
+    TileConst* d_tile_consts = nullptr;
     int arith = 0;
     Variant variant;
     bool dirty = true;
@@ -176,6 +182,52 @@ int batch_commit_pair(go_batch* b) {
     return GO_OK;
 }
 
+// Whether the batch runs the tile kernel: reciprocal quotients on north-up
+// grids, no land told, and members so narrow that the other kernels' whole
+// column blocks and frames cost more than its lower rate per cell.  The tile
+// kernel computes whole tiles of 32 x 16 cells at 56 ns per 1000 cells and step,
+// the column-pair kernel whole blocks of 128 columns, of which 124 are written,
+// and about 3 rows more per 32-row strip at 33 (B200; us per step, tile / best of
+// the others: 60 members of 128^2 68 / 122, 32 of 300^2 185 / 162, 40 of 512^2
+// 589 / 504).
+bool batch_tile(const go_batch* b) {
+    if (!b->auto_launch || b->arith != GO_ARITH_RCP || b->variant.gen_north) return false;
+    double tile = 0.0, pair = 0.0;
+    for (int m = 0; m < b->n; ++m) {
+        const Scheme& k = b->members[m]->k;
+        if (b->members[m]->land_told || !tile_batch_fits(b->args[2 * m]) || !tile_batch_fits(b->args[2 * m + 1]))
+            return false;
+        int gx, gy;
+        tile_batch_dims(k, &gx, &gy);
+        tile += 512.0 * gx * gy;
+        pair += 128.0 * ((k.nx + 123) / 124) * k.ny * (35.0 / 32.0);
+    }
+    return 56.0 * tile < 33.0 * pair;
+}
+
+int batch_commit_tile(go_batch* b) {
+    std::vector<int4> tiles;
+    for (int m = 0; m < b->n; ++m) {
+        int gx, gy;
+        tile_batch_dims(b->members[m]->k, &gx, &gy);
+        for (int y = 0; y < gy; ++y)
+            for (int x = 0; x < gx; ++x) tiles.push_back(make_int4(m, x, y, 0));
+    }
+    cudaFree(b->d_tiles);
+    cudaFree(b->d_tile_consts);
+    b->d_tiles = nullptr;
+    b->d_tile_consts = nullptr;
+    GO_CUDA(cudaMalloc(&b->d_tiles, sizeof(int4) * tiles.size()));
+    GO_CUDA(cudaMemcpy(b->d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice));
+    GO_CUDA(tile_batch_consts(b->args, &b->d_tile_consts));
+    GO_CUDA(cudaMemcpy(b->d_args, b->args.data(), sizeof(StageArgs) * b->args.size(), cudaMemcpyHostToDevice));
+    GO_CUDA(cudaMemcpy(b->d_dt, b->dt.data(), sizeof(float) * b->n, cudaMemcpyHostToDevice));
+    b->ntiles = (int)tiles.size();
+    b->ntiles_frame = 0;
+    b->dirty = false;
+    return GO_OK;
+}
+
 int batch_commit(go_batch* b) {
     if (!b->dirty) return GO_OK;
     for (int m = 0; m < b->n; ++m)
@@ -185,6 +237,8 @@ int batch_commit(go_batch* b) {
     Variant v = b->variant;
     v.shape = b->shape;
     v.rcp = b->arith == GO_ARITH_RCP;
+    b->tile = batch_tile(b);
+    if (b->tile) return batch_commit_tile(b);
     if (go_pair_shape(b->shape)) return batch_commit_pair(b);
     const int width = dispatch_width(v) - 4;
     std::vector<int4> tiles;
@@ -247,7 +301,14 @@ int batch_launch_pair(go_batch* b, int rk_step, cudaStream_t s) {
     return GO_OK;
 }
 
-int batch_launch(go_batch* b, int rk_step, cudaStream_t s) {
+// follows: the launch before it on the stream is a stage of the same call.
+int batch_launch(go_batch* b, int rk_step, cudaStream_t s, bool follows = false) {
+    if (b->tile) {
+        const cudaError_t e = tile_batch_launch(TileBatchReq{b->d_args, b->d_dt, b->d_tile_consts, b->d_tiles, b->ntiles,
+                                                             rk_step, b->members[0]->device, s, follows});
+        if (e != cudaSuccess) return go_fail(GO_ERR_CUDA, "batch stage launch (tiles) failed: %s", cudaGetErrorString(e));
+        return GO_OK;
+    }
     if (go_pair_shape(b->shape)) return batch_launch_pair(b, rk_step, s);
     int grid = b->ntiles;
     if (b->blocks > 0 && b->blocks < grid) grid = b->blocks;
@@ -561,7 +622,32 @@ int go_batch_create(go_domain* const* members, int n, go_batch** out) {
         // 4 members 123 / 125)
         long long cells = 0;
         for (int m = 0; m < n; ++m) cells += (long long)members[m]->k.nx * members[m]->k.ny;
-        if (cells >= kPairAutoBatchCells) b->shape = GO_SHAPE_PAIR;
+        if (cells >= kPairAutoBatchCells) {
+            // strip height by the cost of all members' strips (us per step,
+            // 32 rows / the height taken: 100 members of 195^2 276 / 245, 12
+            // of 700^2 311 / 269, 32 of 300^2 189 / 162)
+            b->shape = GO_SHAPE_PAIR;
+            double best = -1.0;
+            for (int r = 6; r <= 120; ++r) {
+                long long blocks = 0;
+                for (int m = 0; m < n; ++m) {
+                    const Scheme& k = members[m]->k;
+                    blocks += shape_columns(GO_SHAPE_PAIR, k.nx) / shape_block_width(GO_SHAPE_PAIR) *
+                              ((std::max(k.ny - 4, 1) + r - 1) / r);
+                }
+                const double cost = pair_strip_cost(blocks, r);
+                if (best < 0.0 || cost < best) { best = cost; b->rows = r; }
+            }
+        }
+        // with land, 16-row strips of the register-prefetch shape (a seventh of
+        // the corners land in patches; us per step, the choice above / this:
+        // 40 members of 512^2 796 / 685, 32 of 300^2 298 / 229, 8 of 1024^2
+        // 586 / 490, 60 of 128^2 155 / 138)
+        for (int m = 0; m < n; ++m)
+            if (members[m]->land_told) {
+                b->shape = 4;
+                b->rows = 16;
+            }
     }
     for (int m = 0; m < n; ++m) {
         const go_domain* d = members[m];
@@ -602,6 +688,7 @@ int go_batch_destroy(go_batch* b) {
     cudaFree(b->d_args);
     cudaFree(b->d_dt);
     cudaFree(b->d_tiles);
+    cudaFree(b->d_tile_consts);
     cudaFree(b->d_grf);
     cudaFree(b->d_loop);
     cudaFree(b->d_t);
@@ -641,6 +728,7 @@ int go_batch_set_launch(go_batch* b, int shape, int rows_per_block, int blocks) 
     b->shape = shape;
     b->rows = rows_per_block;
     b->blocks = blocks;
+    b->auto_launch = false;
     b->dirty = true;
     drop_graph(b);
     return GO_OK;
@@ -651,6 +739,12 @@ int go_batch_set_arith(go_batch* b, int mode) {
     if (mode != GO_ARITH_EXACT && mode != GO_ARITH_RCP) return go_fail(GO_ERR_INVALID, "arith mode %d", mode);
     b->arith = mode;
     drop_graph(b);
+    // a kernel laid out already that this arithmetic does not run: laid out
+    // anew here, so that the next step allocates nothing
+    if (!b->dirty && batch_tile(b) != b->tile) {
+        b->dirty = true;
+        return batch_commit(b);
+    }
     return GO_OK;
 }
 
@@ -683,9 +777,9 @@ int go_batch_step(go_batch* b, void* stream, int n_steps) {
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     for (int i = 0; i < n_steps; ++i) {
-        rc = batch_launch(b, 0, s);
+        rc = batch_launch(b, 0, s, i > 0);
         if (rc) return rc;
-        rc = batch_launch(b, 1, s);
+        rc = batch_launch(b, 1, s, true);
         if (rc) return rc;
     }
     return GO_OK;

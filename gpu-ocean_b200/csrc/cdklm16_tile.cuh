@@ -635,6 +635,30 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks)
     else tile_one<false>(a, tc, t, sm);
 }
 
+// One batched stage: block i computes tile (member, column, row) of the packed
+// list.  args holds two entries per member (stage 0: h0 -> h1, stage 1: h1 -> h0);
+// dts holds the member's time step, read at launch so a captured graph picks
+// up new values.
+template <bool RIM>
+__device__ __forceinline__ void tile_member(const StageArgs& a, const TileConst& tc, const float* dt,
+                                            const TilePlace& t, TileSmem& sm) {
+    const bool ok = tile_load_fixed<RIM>(a, t, sm);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    tile_stage<RIM>(a, tc, tile_io(a), __ldg(dt), a.rk_step == 1, t, ok, sm);
+}
+
+__global__ void __launch_bounds__(kTileThreads, kTileBlocks)
+    cdklm_tile_batch_kernel(const StageArgs* __restrict__ args, const float* __restrict__ dts,
+                            const TileConst* __restrict__ consts, const int4* __restrict__ tiles, const int rk_step) {
+    TileSmem& sm = *reinterpret_cast<TileSmem*>(tile_smem_raw);
+    const int4 tile = tiles[blockIdx.x];
+    const StageArgs& a = args[2 * tile.x + rk_step];
+    const TilePlace t = tile_place(a.k, tile.y, tile.z);
+    if (warp_uniform(t.rim)) tile_member<true>(a, consts[tile.x], dts + tile.x, t, sm);
+    else tile_member<false>(a, consts[tile.x], dts + tile.x, t, sm);
+}
+
 // n whole steps in one cooperative launch, one tile per block; a: the
 // arguments of stage 0 (h0 -> h1), whose states stage 1 exchanges.  Every block takes
 // part in every grid barrier, and a cooperative launch runs only when all its

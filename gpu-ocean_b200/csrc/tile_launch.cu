@@ -1,8 +1,10 @@
 // Launches of the tile stage kernels (cdklm16_tile.cuh).
 #include <atomic>
+#include <vector>
 
 #include "cdklm16_tile.cuh"
 #include "pair_dispatch.cuh"
+#include "tile_batch.h"
 
 using namespace go;
 
@@ -21,8 +23,29 @@ cudaError_t allow_smem(int device) {
     cudaError_t e = cudaFuncSetAttribute(cdklm_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(cdklm_tile_steps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(cdklm_tile_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
     return e;
+}
+
+// 32-bit byte offsets into every array of a stage.
+bool offsets_fit(const StageArgs& a) {
+    auto fits = [&](int pitch) { return (long long)(a.k.ny + 5) * pitch * 4 < (1LL << 32); };
+    return fits(a.pin) && fits(a.pout) && fits(a.pqn) && fits(a.phi);
+}
+
+cudaLaunchConfig_t tile_config(dim3 grid, cudaStream_t s, cudaLaunchAttribute* attr, bool follows) {
+    attr->id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr->val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kTileThreads);
+    cfg.dynamicSmemBytes = sizeof(TileSmem);
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = follows ? 1 : 0;
+    return cfg;
 }
 
 }  // namespace
@@ -45,10 +68,8 @@ int go_tile_setup(go_domain* d) {
 // 640^2 34.4 / 39.3 but 26.5 / 24.6, 1024^2 68.9 / 78.1 but 63.9 / 52.5.
 bool go_tile_stage(const go_domain* d, const StageArgs& a) {
     const long long cells = (long long)a.k.nx * a.k.ny;
-    // 32-bit byte offsets into every array
-    auto fits = [&](int pitch) { return (long long)(a.k.ny + 5) * pitch * 4 < (1LL << 32); };
     return d->auto_launch && cells < (d->land_told ? kTileLandCells : kTileCells) && d->arith == GO_ARITH_RCP &&
-           !go_general_north(d) && fits(a.pin) && fits(a.pout) && fits(a.pqn) && fits(a.phi);
+           !go_general_north(d) && offsets_fit(a);
 }
 
 // One stage.  follows: the launch before it on the stream is a tile stage of
@@ -57,16 +78,8 @@ bool go_tile_stage(const go_domain* d, const StageArgs& a) {
 // Measured on a B200, us per RK2 step without / with: 64 x 48 12.4 / 9.2,
 // 512^2 20.6 / 16.7, 1024^2 53.4 / 48.5.
 int go_launch_tile(go_domain* d, cudaStream_t s, const StageArgs& a, bool follows) {
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = tile_grid(a.k);
-    cfg.blockDim = dim3(kTileThreads);
-    cfg.dynamicSmemBytes = sizeof(TileSmem);
-    cfg.stream = s;
-    cfg.attrs = attr;
-    cfg.numAttrs = follows ? 1 : 0;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = tile_config(tile_grid(a.k), s, &attr, follows);
     d->stage_launches = 1;
     cudaError_t e = allow_smem(d->device);
     if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, cdklm_tile_kernel, a, tile_const(a.k));
@@ -98,3 +111,32 @@ int go_launch_tile_steps(go_domain* d, cudaStream_t s, const StageArgs& a, int n
     if (e != cudaSuccess) return go_fail(GO_ERR_CUDA, "step launch (tiles) failed: %s", cudaGetErrorString(e));
     return GO_OK;
 }
+
+namespace go {
+
+void tile_batch_dims(const Scheme& k, int* columns, int* rows) {
+    const dim3 g = tile_grid(k);
+    *columns = (int)g.x;
+    *rows = (int)g.y;
+}
+
+bool tile_batch_fits(const StageArgs& a) { return offsets_fit(a); }
+
+cudaError_t tile_batch_consts(const std::vector<StageArgs>& args, TileConst** out) {
+    std::vector<TileConst> h(args.size() / 2);
+    for (size_t m = 0; m < h.size(); ++m) h[m] = tile_const(args[2 * m].k);
+    *out = nullptr;
+    cudaError_t e = cudaMalloc(out, sizeof(TileConst) * h.size());
+    if (e == cudaSuccess) e = cudaMemcpy(*out, h.data(), sizeof(TileConst) * h.size(), cudaMemcpyHostToDevice);
+    return e;
+}
+
+cudaError_t tile_batch_launch(const TileBatchReq& r) {
+    const cudaError_t e = allow_smem(r.device);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = tile_config(dim3(r.ntiles), r.s, &attr, r.follows);
+    return cudaLaunchKernelEx(&cfg, cdklm_tile_batch_kernel, r.args, r.dts, r.consts, r.tiles, r.rk_step);
+}
+
+}  // namespace go

@@ -24,7 +24,7 @@ if __name__ != "__main__":
     if not torch.cuda.is_available():
         pytest.skip("needs a CUDA GPU", allow_module_level=True)
 
-from SWESimulators import CDKLM16, Common, WindStress  # noqa: E402
+from SWESimulators import BatchedEnsemble, CDKLM16, Common, WindStress  # noqa: E402
 
 WALLS, CHANNEL, TORUS = (1, 1, 1, 1), (1, 2, 1, 2), (2, 2, 2, 2)
 # (nx, ny, sides, water, wind, friction)
@@ -88,6 +88,34 @@ def test_tile_kernel_equals_marching_kernel(case):
         assert np.array_equal(a, b, equal_nan=True)
 
 
+# members of a batch share the friction law and the wind kind; narrow grids, so
+# that the batch takes the tile kernel
+BATCHES = [[(32, 16, WALLS, "deep", "uniform", "quadratic"), (33, 17, TORUS, "edge", "uniform", "quadratic"),
+            (120, 50, CHANNEL, "deep", "uniform", "quadratic"), (5, 90, WALLS, "shallow", "uniform", "quadratic")],
+           [(96, 31, CHANNEL, "shallow", "field", "linear"), (64, 64, WALLS, "edge", "field", "linear")]]
+
+
+def _run_batch(cases, graph_steps):
+    ctx = Common.CUDAContext()
+    sims = [_simulator(ctx, c) for c in cases]
+    ens = BatchedEnsemble.BatchedCDKLM16(sims, graph_steps=graph_steps)
+    ens.advance(5)
+    torch.cuda.synchronize()
+    return sims, ens.member_status()
+
+
+@pytest.mark.parametrize("graph_steps", [0, 2])
+@pytest.mark.parametrize("cases", BATCHES, ids=["quadratic", "linear-field"])
+def test_batched_tile_kernel_equals_marching_kernel(cases, graph_steps):
+    sims, status = _run_batch(cases, graph_steps)
+    for sim, word, case in zip(sims, status, cases):
+        march, s_march = _run(case, launch=(4, 4), calls=(1,) * 5)
+        g = sim.gpu_data
+        assert word == s_march
+        for a, b in zip((g.h0, g.hu0, g.hv0, g.h1, g.hu1, g.hv1), march):
+            assert np.array_equal(a.view.cpu().numpy(), b, equal_nan=True)
+
+
 def test_checked_indices_of_the_tile_kernel(tmp_path):
     if not os.path.exists(os.path.join(PKG, "lib", "libgocean_debug.so")):
         pytest.skip("lib/libgocean_debug.so not built")
@@ -100,6 +128,7 @@ def test_checked_indices_of_the_tile_kernel(tmp_path):
         assert int(dbg["status%d" % i]) == status
         for k, a in enumerate(plain):
             assert np.array_equal(dbg["a%d_%d" % (i, k)], a, equal_nan=True)
+    assert not dbg["batch"].any()
 
 
 if __name__ == "__main__":
@@ -109,4 +138,6 @@ if __name__ == "__main__":
         res["status%d" % i] = np.array(status)
         for k, a in enumerate(arrays):
             res["a%d_%d" % (i, k)] = a
+    # GO_STATUS_BOUNDS of the batches' members
+    res["batch"] = np.array([w & 8 for cases in BATCHES for w in _run_batch(cases, 0)[1]])
     np.savez(sys.argv[1], **res)
