@@ -100,8 +100,9 @@ class BatchedCDKLM16:
         # later work on a member's own stream waits for the batch's
         if getattr(self, "_owned", False):
             return
+        done = self.stream.record_event()    # one event for all members
         for s in self.sims:
-            s.gpu_stream.wait_stream(self.stream)
+            s.gpu_stream.wait_event(done)
 
     def _first_step_bc(self):
         # on the batch stream, after _sync_members
@@ -153,8 +154,10 @@ class BatchedCDKLM16:
         for s in self.sims:
             key = (float(s.t), float(np.float32(s.dt)))
             if key not in sums:
-                steps = np.full(int(n_steps), np.float64(np.float32(s.dt)))
-                sums[key] = float(np.cumsum(np.concatenate([[np.float64(s.t)], steps]))[-1])
+                t, step = key
+                for _ in range(int(n_steps)):
+                    t += step
+                sums[key] = t
             s.t = sums[key]
             s.num_iterations += n_steps
 

@@ -236,7 +236,15 @@ class CDKLM16(Simulator.Simulator):
         t_now = 0.0
         time_varying_wind = len(self.wind_stress.t) > 1
         pending_n, pending_dt, pending_w = 0, None, None
+        one_by_one = self.hasDrifters or time_varying_wind or open_bc or perturb
         while t_now < t_end:
+            if pending_n and not update_dt and not one_by_one and pending_w == 1.0:
+                # one wind field at its full weight and nothing between the
+                # steps: only the step length can change from here on
+                n, t_now = self._whole_steps(pending_dt, t_now, t_end)
+                pending_n += n
+                if t_now >= t_end:
+                    break
             if update_dt:
                 if pending_n:
                     self._launch_steps(pending_n, pending_dt, pending_w)
@@ -244,13 +252,12 @@ class CDKLM16(Simulator.Simulator):
                 self.updateDt()
             local_dt = np.float32(min(self.dt, np.float32(t_end - t_now)))
             wind_t = np.float32(self.update_wind_stress())
-            if pending_n and (local_dt != pending_dt or wind_t != pending_w or time_varying_wind
-                              or self.hasDrifters or open_bc or perturb):
+            if pending_n and (local_dt != pending_dt or wind_t != pending_w or one_by_one):
                 self._launch_steps(pending_n, pending_dt, pending_w)
                 pending_n = 0
             pending_n += 1
             pending_dt, pending_w = local_dt, wind_t
-            if self.hasDrifters or time_varying_wind or open_bc or perturb:
+            if one_by_one:
                 # one launch per step: the drifters move between steps, the
                 # wind or the exterior solution of this step's time, the
                 # model error perturbs each step's result before its
@@ -271,6 +278,27 @@ class CDKLM16(Simulator.Simulator):
         if self.write_netcdf and write_now:
             self.sim_writer.writeTimestep(self)
         return self.t
+
+    def _whole_steps(self, dt, t_now, t_end):
+        """Counts and accounts for the steps of length dt (float32) that the
+        step loop takes next: while float32(min(self.dt, float32(t_end -
+        t_now))) is dt, with t_now and self.t advancing by float64(dt) each
+        step, in the loop's own float64 sums.  The time left is compared in
+        float64 and rounded as the loop does only when it is near dt."""
+        step, limit = float(dt), float(self.dt)
+        if np.float32(limit) != dt:
+            return 0, t_now
+        t, now, end, n = float(self.t), float(t_now), float(t_end), 0
+        near = max(step, limit) * (1.0 + 1.0e-6)
+        while now < end:
+            if end - now < near and np.float32(min(self.dt, np.float32(end - now))) != dt:
+                break
+            t += step
+            now += step
+            n += 1
+        self.t = np.float64(t)
+        self.num_iterations += n
+        return n, now
 
     def drifterStep(self, dt):
         """Advances the attached drifters through the new state

@@ -70,6 +70,9 @@ class Simulator(object):
         next wind to the kernel and returns the time-interpolation weight."""
         domain = domain if domain is not None else self._domain
         ws = self.wind_stress
+        if len(ws.t) == 1 and self.wind_stress_timestamps.get("cdklm") == [ws.t[0], ws.t[0]]:
+            # one wind field, bound already: the weight of the general form below
+            return max(0.0, min(1.0, (self.t - ws.t[0]) / 1.0e-10))
         t0_index, t1_index = self._wind_interval()
         new_t0, new_t1 = ws.t[t0_index], ws.t[t1_index]
         old = self.wind_stress_timestamps.get("cdklm")
