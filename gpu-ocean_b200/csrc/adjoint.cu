@@ -28,6 +28,14 @@
 // velocities, wave speeds) keeps the forward kernel's rounding: products that
 // feed a sum are written with __fmul_rn so that they are never contracted.
 //
+// Quotients are products with rcp.approx (the forward's own quotients, so the
+// branches are the forward's), each reciprocal taken once per cell or face, and
+// a slope's adjoint is scattered as two products (SlopeAdj): both launch forms
+// are bound by instruction issue, and of some 2000 instructions per cell and
+// stage a fifth were division sequences.  Stage adjoint on a B200, before and
+// after, us: 512^2 37.5 / 34.6 (tile form), 768^2 68.2 / 61.1, 1024^2 116 / 90
+// (marching form), 2048^2 369 / 295.
+//
 // Two launch forms compute the same adjoint.  Tile form: one CTA per output
 // tile of TX x TY cells of the ghost-inclusive grid.  The forward state of the tile plus a 3-cell halo is recomputed in
 // shared memory; the adjoint then flows output -> fluxes -> slopes -> cell
@@ -109,22 +117,28 @@ __device__ __forceinline__ int mm_branch(float b, float c, float f) {
     return af > 0.0f ? kBrFwd : kBrZero;
 }
 
-// d slope / d value at position pos (-1 left, 0 centre, +1 right) for the
-// minmod of theta*(c-l), (r-l)/2, theta*(r-c).
-__device__ __forceinline__ float slope_coef(int br, int pos, float theta) {
-    if (br == kBrBack) return pos < 0 ? -theta : (pos == 0 ? theta : 0.0f);
-    if (br == kBrCent) return pos < 0 ? -0.5f : (pos == 0 ? 0.0f : 0.5f);
-    if (br == kBrFwd) return pos < 0 ? 0.0f : (pos == 0 ? -theta : theta);
-    return 0.0f;
+// minmod_raw's value for the branch mm_branch returns.
+__device__ __forceinline__ float mm_value(int br, float b, float c, float f) {
+    return br == kBrBack ? b : (br == kBrCent ? c : (br == kBrFwd ? f : 0.0f));
+}
+// The slope of l, c, r (minmod of theta (c - l), (r - l) / 2, theta (r - c)) and its branch.
+__device__ __forceinline__ float mm_slope(float l, float c, float r, float theta, int& br) {
+    const float b = (c - l) * theta, m = (r - l) * 0.5f, f = (r - c) * theta;
+    br = mm_branch(b, m, f);
+    return mm_value(br, b, m, f);
 }
 
-// d (sum of the Coriolis terms inside K or L) / d f*v at position pos:
-// backward (fc + fl), central ((fr + 2 fc) + fl)/2... scaled by theta*g or g/2.
-__device__ __forceinline__ float pot_coef(int br, int pos, float theta_g, float half_g) {
-    if (br == kBrBack) return pos > 0 ? 0.0f : theta_g;
-    if (br == kBrCent) return pos == 0 ? 2.0f * half_g : half_g;
-    if (br == kBrFwd) return pos < 0 ? 0.0f : theta_g;
-    return 0.0f;
+// A slope is p-weight (c - l) + q-weight (r - c): (wide, 0) on the backward
+// branch, (half, half) on the central and (0, wide) on the forward one, with
+// wide = theta, half = 1/2 (times g for the potentials K and L).  For the
+// adjoint lam of the slope, p and q are lam times those: its left cell
+// receives -p, the cell itself p - q and its right cell q, and the Coriolis
+// products of a potential (backward fc + fl, central fr + 2 fc + fl, forward
+// fr + fc) p, p + q and q.
+struct SlopeAdj { float p, q; };
+__device__ __forceinline__ SlopeAdj slope_adj(int br, float lam, float wide, float half) {
+    const float c = br == kBrCent ? half : 0.0f;
+    return SlopeAdj{lam * (br == kBrBack ? wide : c), lam * (br == kBrFwd ? wide : c)};
 }
 
 __device__ __forceinline__ float flip(bool f) { return f ? -1.0f : 1.0f; }
@@ -162,7 +176,8 @@ __device__ __forceinline__ int adj_prim(float qe, float qu, float qv, float sw, 
         v = desingularize(h, qv, k.desing_eps);
         return kCellDesing;
     }
-    e = qe; u = qu / h; v = qv / h;
+    const float rh = rcp_approx_f(h);     // the forward's quotients, never contracted with a later sum
+    e = qe; u = __fmul_rn(qu, rh); v = __fmul_rn(qv, rh);
     return kCellWet;
 }
 
@@ -175,12 +190,12 @@ __device__ __forceinline__ Trip3 adj_prim_vjp(int cls, float qe, float u, float 
     const float s4 = ((sw + nw) + se) + ne;
     const float Bm = LAND ? cell_bm(sw, nw, se, ne, s4, k) : __fmul_rn(s4, 0.25f);
     const float h = qe + Bm;
-    float D = h, gD = 1.0f / h;                 // u = hu / D(h): du/dh = -u D'(h) / D
+    float rD = rcp_approx_f(h), gD = rD;        // u = hu / D(h): du/dh = -u D'(h) / D
     if (cls == kCellDesing) {
-        D = desing_den(h, k.desing_eps);
-        gD = desing_den_dh(h, k.desing_eps) / D;
+        rD = rcp_approx_f(desing_den(h, k.desing_eps));
+        gD = desing_den_dh(h, k.desing_eps) * rD;
     }
-    return Trip3{l0 - (l1 * u + l2 * v) * gD, l1 / D, l2 / D};
+    return Trip3{l0 - (l1 * u + l2 * v) * gD, l1 * rD, l2 * rD};
 }
 
 struct CuGrad { float hm, um, vm, hp, up, vp; };
@@ -210,7 +225,7 @@ __device__ __forceinline__ CuGrad cu_vjp(float hm, float um, float vm, float hp,
     const float am = fminf(fminf(a1, a2), 0.0f);
     const float ap = fmaxf(fmaxf(b1, b2), 0.0f);
     if (fabsf(ap - am) < k.flux_slope_eps) return g;
-    const float id = 1.0f / (ap - am);
+    const float id = rcp_approx_f(ap - am);
     const float dh = hp - hm, dF0 = Fp0 - Fm0;
     const float F0 = ((ap * Fm0 - am * Fp0) + ap * am * dh) * id;
     const float F1 = ((ap * Fm1 - am * Fp1) + ap * am * dF0) * id;
@@ -231,12 +246,12 @@ __device__ __forceinline__ CuGrad cu_vjp(float hm, float um, float vm, float hp,
         if (a1 <= a2) { lumw += lam; lcm -= lam; } else { lupw += lam; lcp -= lam; }
     }
     if (wp) {
-        g.hp += lFp0 * up + lFp1 * (up * up + k.g * hp) + lFp2 * up * vp + lcp * (0.5f * k.g / cp);
+        g.hp += lFp0 * up + lFp1 * (up * up + k.g * hp) + lFp2 * up * vp + lcp * (k.half_g * rcp_approx_f(cp));
         g.up += lupw + lFp0 * hp + lFp1 * 2.0f * hp * up + lFp2 * hp * vp;
         g.vp += lFp2 * hp * up;
     }
     if (wm) {
-        g.hm += lFm0 * um + lFm1 * (um * um + k.g * hm) + lFm2 * um * vm + lcm * (0.5f * k.g / cm);
+        g.hm += lFm0 * um + lFm1 * (um * um + k.g * hm) + lFm2 * um * vm + lcm * (k.half_g * rcp_approx_f(cm));
         g.um += lumw + lFm0 * hm + lFm1 * 2.0f * hm * um + lFm2 * hm * vm;
         g.vm += lFm2 * hm * um;
     }
@@ -297,7 +312,7 @@ __global__ void __launch_bounds__(NT, MINB) cdklm_adjoint_stage_kernel(const Adj
     const int ox = blockIdx.x * TX - HALO, oy = blockIdx.y * TY - HALO;
     const int tid = threadIdx.x;
     const bool wallN = k.bcN == kWall, wallS = k.bcS == kWall, wallE = k.bcE == kWall, wallW = k.bcW == kWall;
-    const float inv2g = 1.0f / k.two_g;
+    const float inv2g = rcp_approx_f(k.two_g), inv_dx = rcp_approx_f(k.dx), inv_dy = rcp_approx_f(k.dy);
     auto RI = [](int ry, int rx) { return ry * RXS + rx; };                 // region
     auto XI = [](int ry, int rx) { return (ry - HALO) * RXS + rx; };        // tile rows
     auto YI = [](int ry, int rx) { return ry * TX + (rx - HALO); };         // tile columns
@@ -376,23 +391,22 @@ __global__ void __launch_bounds__(NT, MINB) cdklm_adjoint_stage_kernel(const Adj
         const float vl = S.R2[q - 1], vc = S.R2[q], vr = S.R2[q + 1];
         const float el = S.R0[q - 1], ec = S.R0[q], er = S.R0[q + 1];
         const int xi = XI(ry, rx);
-        S.Ux[xi] = minmod_slope(ul, uc, ur, k.theta);
-        S.Vx[xi] = minmod_slope(vl, vc, vr, k.theta);
-        const int bu = mm_branch((uc - ul) * k.theta, (ur - ul) * 0.5f, (ur - uc) * k.theta);
-        const int bv = mm_branch((vc - vl) * k.theta, (vr - vl) * 0.5f, (vr - vc) * k.theta);
+        int bu, bv;
+        S.Ux[xi] = mm_slope(ul, uc, ur, k.theta, bu);
+        S.Vx[xi] = mm_slope(vl, vc, vr, k.theta, bv);
         const float fvl = (vl * flip((wallW && i - 1 < 2) || (wallE && i - 1 > nx + 1))) * fJ;
         const float fvc = (vc * flip((wallW && i < 2) || (wallE && i > nx + 1))) * fJ;
         const float fvr = (vr * flip((wallW && i + 1 < 2) || (wallE && i + 1 > nx + 1))) * fJ;
         const float bw = k.theta_g * ((ec - el) - __fmul_rn(k.V, fvc + fvl));
         const float ce = k.half_g * ((er - el) - __fmul_rn(k.V, (fvr + __fmul_rn(2.0f, fvc)) + fvl));
         const float fw = k.theta_g * ((er - ec) - __fmul_rn(k.V, fvc + fvr));
-        const float Kraw = minmod_raw(bw, ce, fw);
         const int bk = mm_branch(bw, ce, fw);
+        const float Kraw = mm_value(bk, bw, ce, fw);
         const float dxfv = __fmul_rn(k.dx * fJ, vc * flip((wallW && i < 2) || (wallE && i > nx + 2)));
         const float Hw = 0.5f * (HI(ry, rx) + HI(ry + 1, rx));
         const float He = 0.5f * (HI(ry, rx + 1) + HI(ry + 1, rx + 1));
-        const float hw = (ec + Hw) - (Kraw + dxfv) / k.two_g;
-        const float he = (ec + He) + (Kraw + dxfv) / k.two_g;
+        const float hw = (ec + Hw) - __fmul_rn(Kraw + dxfv, inv2g);
+        const float he = (ec + He) + __fmul_rn(Kraw + dxfv, inv2g);
         float K = Kraw;
         int ba = kAdjNone;
         if (!(hw > 0.0f)) { K = -dxfv + __fmul_rn(k.two_g, ec + Hw); ba = kAdjA; }
@@ -409,23 +423,22 @@ __global__ void __launch_bounds__(NT, MINB) cdklm_adjoint_stage_kernel(const Adj
         const float vl = S.R2[q - RXS], vc = S.R2[q], vr = S.R2[q + RXS];
         const float el = S.R0[q - RXS], ec = S.R0[q], er = S.R0[q + RXS];
         const int yi = YI(ry, rx);
-        S.Uy[yi] = minmod_slope(ul, uc, ur, k.theta);
-        S.Vy[yi] = minmod_slope(vl, vc, vr, k.theta);
-        const int bu = mm_branch((uc - ul) * k.theta, (ur - ul) * 0.5f, (ur - uc) * k.theta);
-        const int bv = mm_branch((vc - vl) * k.theta, (vr - vl) * 0.5f, (vr - vc) * k.theta);
+        int bu, bv;
+        S.Uy[yi] = mm_slope(ul, uc, ur, k.theta, bu);
+        S.Vy[yi] = mm_slope(vl, vc, vr, k.theta, bv);
         const float ful = (ul * flip((wallS && j - 1 < 2) || (wallN && j - 1 > ny + 1))) * S.f[ry - 1];
         const float fuc = (uc * flip((wallS && j < 2) || (wallN && j > ny + 1))) * S.f[ry];
         const float fur = (ur * flip((wallS && j + 1 < 2) || (wallN && j + 1 > ny + 1))) * S.f[ry + 1];
         const float bw = k.theta_g * ((ec - el) + __fmul_rn(k.U, fuc + ful));
         const float ce = k.half_g * ((er - el) + __fmul_rn(k.U, (fur + __fmul_rn(2.0f, fuc)) + ful));
         const float fw = k.theta_g * ((er - ec) + __fmul_rn(k.U, fuc + fur));
-        const float Lraw = minmod_raw(bw, ce, fw);
         const int bl = mm_branch(bw, ce, fw);
+        const float Lraw = mm_value(bl, bw, ce, fw);
         const float dyfu = __fmul_rn(k.dy * S.f[ry], uc * flip((wallS && j < 2) || (wallN && j > ny + 2)));
         const float Hs = 0.5f * (HI(ry, rx) + HI(ry, rx + 1));
         const float Hn = 0.5f * (HI(ry + 1, rx) + HI(ry + 1, rx + 1));
-        const float hs = (ec + Hs) - (Lraw - dyfu) / k.two_g;
-        const float hn = (ec + Hn) + (Lraw - dyfu) / k.two_g;
+        const float hs = (ec + Hs) - __fmul_rn(Lraw - dyfu, inv2g);
+        const float hn = (ec + Hn) + __fmul_rn(Lraw - dyfu, inv2g);
         float L = Lraw;
         int ba = kAdjNone;
         if (!(hs > 0.0f)) { L = dyfu + __fmul_rn(k.two_g, ec + Hs); ba = kAdjA; }
@@ -485,34 +498,37 @@ __global__ void __launch_bounds__(NT, MINB) cdklm_adjoint_stage_kernel(const Adj
             const float h = e + Hm;
             const bool wet = h > k.cutoff;
             const float hu = wet ? u * h : 0.0f, hv = wet ? v * h : 0.0f;
-            float Cf = 0.0f, sq = 0.0f, uw = 0.0f, vw = 0.0f, Dn = h;
+            float Cf = 0.0f, sq = 0.0f, uw = 0.0f, vw = 0.0f, Dn = h, rDn = 0.0f;
             if (FRIC == kFricQuad) {
                 // below desing_eps the speed and C are desingularised (CDKLM16_kernel.cu:884-900)
                 if (h < k.desing_eps) Dn = desing_den(h, k.desing_eps);
-                uw = hu / Dn; vw = hv / Dn;
+                rDn = rcp_approx_f(Dn);
+                uw = hu * rDn; vw = hv * rDn;
                 sq = sqrtf(uw * uw + vw * vw);
-                Cf = (a.dt * k.r * sq) / Dn;
+                Cf = a.dt * k.r * sq * rDn;
             } else if (FRIC == kFricLinear) {
-                Cf = (k.two_r * a.dt) / h;
+                rDn = rcp_approx_f(h);
+                Cf = k.two_r * a.dt * rDn;
             }
             const float w = STAGE1 ? 0.5f : 1.0f;
-            const float iD = 1.0f / (1.0f + w * Cf);
+            const float iD = rcp_approx_f(1.0f + w * Cf);
             const float lL1 = w * a.dt * le, lL2 = w * a.dt * lu * iD, lL3 = w * a.dt * lv * iD;
             S.LL0[r] = lL1; S.LL1[r] = lL2; S.LL2[r] = lL3;
             if (!tile) continue;        // the own-cell terms are needed for the tile's cells only
             float lhu = w * lu * iD, lhv = w * lv * iD, leta = w * le, lh = 0.0f;
             const float lCf = -w * (lu * oU[it] + lv * oV[it]) * iD;
             if (FRIC == kFricQuad) {
-                const float ls = lCf * a.dt * k.r / Dn;
-                float lD = -lCf * Cf / Dn;
+                const float ls = lCf * a.dt * k.r * rDn;
+                float lD = -lCf * Cf * rDn;
                 if (sq > 0.0f) {
-                    const float luw = ls * uw / sq, lvw = ls * vw / sq;
-                    lhu += luw / Dn; lhv += lvw / Dn;
-                    lD -= (luw * uw + lvw * vw) / Dn;
+                    const float rsq = ls * rcp_approx_f(sq) * rDn;
+                    const float luw = rsq * uw, lvw = rsq * vw;
+                    lhu += luw; lhv += lvw;
+                    lD -= luw * uw + lvw * vw;
                 }
                 lh += (h < k.desing_eps) ? lD * desing_den_dh(h, k.desing_eps) : lD;
             } else if (FRIC == kFricLinear) {
-                lh -= lCf * Cf / h;
+                lh -= lCf * Cf * rDn;
             }
             const float fc = S.f[ry];
             if (h >= k.cutoff && e != kDryFlag) {
@@ -520,7 +536,7 @@ __global__ void __launch_bounds__(NT, MINB) cdklm_adjoint_stage_kernel(const Adj
                 const float Hy = 0.5f * (HI(ry + 1, rx) + HI(ry + 1, rx + 1)) - 0.5f * (HI(ry, rx) + HI(ry, rx + 1));
                 lhv += fc * lL2;
                 lhu -= fc * lL3;
-                leta += lL2 * k.g * Hx / k.dx + lL3 * k.g * Hy / k.dy;
+                leta += lL2 * k.g * Hx * inv_dx + lL3 * k.g * Hy * inv_dy;
                 if (a.wx) {
                     const size_t wo = (size_t)(j - 2) * a.pw + (i - 2);
                     a.wx[wo] = wX[it] + lL2;
@@ -566,12 +582,12 @@ __global__ void __launch_bounds__(NT, MINB) cdklm_adjoint_stage_kernel(const Adj
                 const float Rpu = S.R1[p] - __fmul_rn(0.5f, S.Ux[xp]), Rpv = S.R2[p] - __fmul_rn(0.5f, S.Vx[xp]);
                 const float fm = flip(wallW && ip == 2), fp = flip(wallE && ip == nx + 2);
                 const float Hf = 0.5f * (HI(ry, rx + 1) + HI(ry + 1, rx + 1));
-                const float Ep = (S.R0[p] + Hf) - (S.Kx[xp] + __fmul_rn(k.dx * fJ, S.R2[p] * fp)) / k.two_g;
-                const float Em = (S.R0[m] + Hf) + (S.Kx[xm] + __fmul_rn(k.dx * fJ, S.R2[m] * fm)) / k.two_g;
+                const float Ep = (S.R0[p] + Hf) - __fmul_rn(S.Kx[xp] + __fmul_rn(k.dx * fJ, S.R2[p] * fp), inv2g);
+                const float Em = (S.R0[m] + Hf) + __fmul_rn(S.Kx[xm] + __fmul_rn(k.dx * fJ, S.R2[m] * fm), inv2g);
                 const float hp = fmaxf(Ep, 0.0f), hm = fmaxf(Em, 0.0f);
-                const float l0 = (S.LL0[p] - S.LL0[m]) / k.dx;
-                const float l1 = (S.LL1[p] - S.LL1[m]) / k.dx;
-                const float l2 = (S.LL2[p] - S.LL2[m]) / k.dx;
+                const float l0 = (S.LL0[p] - S.LL0[m]) * inv_dx;
+                const float l1 = (S.LL1[p] - S.LL1[m]) * inv_dx;
+                const float l2 = (S.LL2[p] - S.LL2[m]) * inv_dx;
                 const CuGrad g = cu_vjp(hm, Rmu, Rmv, hp, Rpu, Rpv, l0, l1, l2, k);
                 if (Ep > 0.0f) {
                     S.Ax0[xp] += g.hp;
@@ -602,13 +618,13 @@ __global__ void __launch_bounds__(NT, MINB) cdklm_adjoint_stage_kernel(const Adj
                 const float fm = flip(wallS && jp == 2), fp = flip(wallN && jp == ny + 2);
                 const float fpr = S.f[ry + 1], fmr = S.f[ry];
                 const float Hf = 0.5f * (HI(ry + 1, rx) + HI(ry + 1, rx + 1));
-                const float Ep = (S.R0[p] + Hf) - (S.Ly[yp] - __fmul_rn(k.dy * fpr, S.R1[p] * fp)) / k.two_g;
-                const float Em = (S.R0[m] + Hf) + (S.Ly[ym] - __fmul_rn(k.dy * fmr, S.R1[m] * fm)) / k.two_g;
+                const float Ep = (S.R0[p] + Hf) - __fmul_rn(S.Ly[yp] - __fmul_rn(k.dy * fpr, S.R1[p] * fp), inv2g);
+                const float Em = (S.R0[m] + Hf) + __fmul_rn(S.Ly[ym] - __fmul_rn(k.dy * fmr, S.R1[m] * fm), inv2g);
                 const float hp = fmaxf(Ep, 0.0f), hm = fmaxf(Em, 0.0f);
                 // G = CU(hm, v, u | hp, v, u) with outputs (G0, G2, G1)
-                const float l0 = (S.LL0[p] - S.LL0[m]) / k.dy;
-                const float l1 = (S.LL1[p] - S.LL1[m]) / k.dy;
-                const float l2 = (S.LL2[p] - S.LL2[m]) / k.dy;
+                const float l0 = (S.LL0[p] - S.LL0[m]) * inv_dy;
+                const float l1 = (S.LL1[p] - S.LL1[m]) * inv_dy;
+                const float l2 = (S.LL2[p] - S.LL2[m]) * inv_dy;
                 const CuGrad g = cu_vjp(hm, Rmv, Rmu, hp, Rpv, Rpu, l0, l2, l1, k);
                 if (Ep > 0.0f) {
                     S.Ay0[yp] += g.hp;
@@ -666,28 +682,25 @@ __global__ void __launch_bounds__(NT, MINB) cdklm_adjoint_stage_kernel(const Adj
         float l1 = S.Ax1[xq] + S.Ay1[yq];
         float l2 = S.Ax2[xq] + S.Ay2[yq];
         float lfv = 0.0f, lfu = 0.0f;
-#pragma unroll
-        for (int o = -1; o <= 1; ++o) {
-            const int pos = -o;       // position of this cell in the stencil of slope cell q+o
-            const uint32_t bxo = S.bx[xq + o];
-            if (br_has(bxo)) {
-                l1 += S.AUx[xq + o] * slope_coef(br_u(bxo), pos, k.theta);
-                l2 += S.AVx[xq + o] * slope_coef(br_v(bxo), pos, k.theta);
-                const float lk = S.AKx[xq + o];
-                const int bk = br_k(bxo);
-                l0 += lk * k.g * slope_coef(bk, pos, k.theta);
-                lfv -= lk * k.V * pot_coef(bk, pos, k.theta_g, k.half_g);
-            }
-            const uint32_t byo = S.by[yq + o * TX];
-            if (br_has(byo)) {
-                l1 += S.AUy[yq + o * TX] * slope_coef(br_u(byo), pos, k.theta);
-                l2 += S.AVy[yq + o * TX] * slope_coef(br_v(byo), pos, k.theta);
-                const float ll = S.ALy[yq + o * TX];
-                const int bl = br_k(byo);
-                l0 += ll * k.g * slope_coef(bl, pos, k.theta);
-                lfu += ll * k.U * pot_coef(bl, pos, k.theta_g, k.half_g);
-            }
-        }
+        // slope cells left of, at and right of this one (a cell without a slope has the zero branch)
+        auto gather = [&](const float* AU, const float* AV, const float* AK, const uint16_t* code, int o, int step,
+                          float UV, float& lf) {
+            const uint32_t bl = code[o - step], bc = code[o], br = code[o + step];
+            auto sum = [&](const float* A, auto field, float wide, float half, float& pq) {
+                const SlopeAdj c = slope_adj(field(bc), A[o], wide, half);
+                const float ql = slope_adj(field(bl), A[o - step], wide, half).q;
+                const float pr = slope_adj(field(br), A[o + step], wide, half).p;
+                pq = (c.p + c.q) + (ql + pr);
+                return (c.p - c.q) + (ql - pr);
+            };
+            float pq;
+            l1 += sum(AU, [](uint32_t c) { return br_u(c); }, k.theta, 0.5f, pq);
+            l2 += sum(AV, [](uint32_t c) { return br_v(c); }, k.theta, 0.5f, pq);
+            l0 += sum(AK, [](uint32_t c) { return br_k(c); }, k.theta_g, k.half_g, pq);
+            lf = UV * pq;
+        };
+        gather(S.AUx, S.AVx, S.AKx, S.bx, xq, 1, -k.V, lfv);
+        gather(S.AUy, S.AVy, S.ALy, S.by, yq, TX, k.U, lfu);
         l2 += lfv * S.f[ry] * flip((wallW && i < 2) || (wallE && i > nx + 1));
         l1 += lfu * S.f[ry] * flip((wallS && j < 2) || (wallN && j > ny + 1));
         const Trip3 lq = adj_prim_vjp<LAND>((S.bx[xq] >> 9) & 3, S.R0[q], S.R1[q], S.R2[q], HI(ry, rx), HI(ry + 1, rx),
@@ -726,10 +739,9 @@ template <int BW>
 struct MarchBufs {
     float e[BW], u[BW], v[BW];              // state of the row
     float su[BW], sv[BW], sK[BW];           // x slopes of the row
-    uint32_t code[BW];                      // their branch codes
     float l0[BW], l1[BW], l2[BW];           // lambda_L of the row
     float pe[BW], pu[BW], pv[BW], pK[BW], pux[BW], pvx[BW];   // face (t, t+1) -> cell t+1
-    float gu[BW], gv[BW], gK[BW];           // x-slope adjoints after the adjustment
+    float gup[BW], guq[BW], gvp[BW], gvq[BW], gKp[BW], gKq[BW];   // x-slope adjoints (SlopeAdj)
 };
 
 template <int BW, int FRIC, bool STAGE1, bool EDGE, bool LAND>
@@ -747,7 +759,7 @@ __device__ __forceinline__ void adjoint_march_strip(const AdjArgs& a, const int 
     const bool col_ok = !EDGE || (i >= 0 && i < nx + 4);
     const bool col_int = !EDGE || (i >= 2 && i < nx + 2);
     const bool writer = t >= 3 && t < BW - 3 && col_ok;
-    const float inv2g = 1.0f / k.two_g;
+    const float inv2g = rcp_approx_f(k.two_g), inv_dx = rcp_approx_f(k.dx), inv_dy = rcp_approx_f(k.dy);
     // column mirror of the load and sign of hu
     int si = i;
     float shu = 1.0f;
@@ -809,23 +821,22 @@ __device__ __forceinline__ void adjoint_march_strip(const AdjArgs& a, const int 
                       const Cor& clo, const Cor& chi) -> SlopeC {
         SlopeC s{0.0f, 0.0f, 0.0f, 0u};
         if (EDGE && !(col_int && r >= 1 && r <= ny + 2)) return s;
-        s.u = minmod_slope(pl.u, pc.u, pr.u, k.theta);
-        s.v = minmod_slope(pl.v, pc.v, pr.v, k.theta);
-        const int bu = mm_branch((pc.u - pl.u) * k.theta, (pr.u - pl.u) * 0.5f, (pr.u - pc.u) * k.theta);
-        const int bv = mm_branch((pc.v - pl.v) * k.theta, (pr.v - pl.v) * 0.5f, (pr.v - pc.v) * k.theta);
+        int bu, bv;
+        s.u = mm_slope(pl.u, pc.u, pr.u, k.theta, bu);
+        s.v = mm_slope(pl.v, pc.v, pr.v, k.theta, bv);
         const float ful = (pl.u * uflip_ly(r - 1)) * fl;
         const float fuc = (pc.u * uflip_ly(r)) * fc;
         const float fur = (pr.u * uflip_ly(r + 1)) * fr;
         const float bw = k.theta_g * ((pc.e - pl.e) + __fmul_rn(k.U, fuc + ful));
         const float ce = k.half_g * ((pr.e - pl.e) + __fmul_rn(k.U, (fur + __fmul_rn(2.0f, fuc)) + ful));
         const float fw = k.theta_g * ((pr.e - pc.e) + __fmul_rn(k.U, fuc + fur));
-        const float Lraw = minmod_raw(bw, ce, fw);
         const int bl = mm_branch(bw, ce, fw);
+        const float Lraw = mm_value(bl, bw, ce, fw);
         const float dyfu = __fmul_rn(k.dy * fc, pc.u * flip(EDGE && ((wallS && r < 2) || (wallN && r > ny + 2))));
         const float Hs = 0.5f * (clo.a + clo.b);
         const float Hn = 0.5f * (chi.a + chi.b);
-        const float hs = (pc.e + Hs) - (Lraw - dyfu) / k.two_g;
-        const float hn = (pc.e + Hn) + (Lraw - dyfu) / k.two_g;
+        const float hs = (pc.e + Hs) - __fmul_rn(Lraw - dyfu, inv2g);
+        const float hn = (pc.e + Hn) + __fmul_rn(Lraw - dyfu, inv2g);
         float L = Lraw;
         int ba = kAdjNone;
         if (!(hs > 0.0f)) { L = dyfu + __fmul_rn(k.two_g, pc.e + Hs); ba = kAdjA; }
@@ -847,32 +858,35 @@ __device__ __forceinline__ void adjoint_march_strip(const AdjArgs& a, const int 
         const float h = p.e + Hm;
         const bool wet = h > k.cutoff;
         const float hu = wet ? p.u * h : 0.0f, hv = wet ? p.v * h : 0.0f;
-        float Cf = 0.0f, sq = 0.0f, uw = 0.0f, vw = 0.0f, Dn = h;
+        float Cf = 0.0f, sq = 0.0f, uw = 0.0f, vw = 0.0f, Dn = h, rDn = 0.0f;
         if (FRIC == kFricQuad) {
             // below desing_eps the speed and C are desingularised (CDKLM16_kernel.cu:884-900)
             if (h < k.desing_eps) Dn = desing_den(h, k.desing_eps);
-            uw = hu / Dn; vw = hv / Dn;
+            rDn = rcp_approx_f(Dn);
+            uw = hu * rDn; vw = hv * rDn;
             sq = sqrtf(uw * uw + vw * vw);
-            Cf = (a.dt * k.r * sq) / Dn;
+            Cf = a.dt * k.r * sq * rDn;
         } else if (FRIC == kFricLinear) {
-            Cf = (k.two_r * a.dt) / h;
+            rDn = rcp_approx_f(h);
+            Cf = k.two_r * a.dt * rDn;
         }
         const float w = STAGE1 ? 0.5f : 1.0f;
-        const float iD = 1.0f / (1.0f + w * Cf);
+        const float iD = rcp_approx_f(1.0f + w * Cf);
         const Trip LL{w * a.dt * lE, w * a.dt * lU * iD, w * a.dt * lV * iD};
         float lhu = w * lU * iD, lhv = w * lV * iD, leta = w * lE, lh = 0.0f;
         const float lCf = -w * (lU * in.ou + lV * in.ov) * iD;
         if (FRIC == kFricQuad) {
-            const float ls = lCf * a.dt * k.r / Dn;
-            float lD = -lCf * Cf / Dn;
+            const float ls = lCf * a.dt * k.r * rDn;
+            float lD = -lCf * Cf * rDn;
             if (sq > 0.0f) {
-                const float luw = ls * uw / sq, lvw = ls * vw / sq;
-                lhu += luw / Dn; lhv += lvw / Dn;
-                lD -= (luw * uw + lvw * vw) / Dn;
+                const float rsq = ls * rcp_approx_f(sq) * rDn;
+                const float luw = rsq * uw, lvw = rsq * vw;
+                lhu += luw; lhv += lvw;
+                lD -= luw * uw + lvw * vw;
             }
             lh += (h < k.desing_eps) ? lD * desing_den_dh(h, k.desing_eps) : lD;
         } else if (FRIC == kFricLinear) {
-            lh -= lCf * Cf / h;
+            lh -= lCf * Cf * rDn;
         }
         const bool out_cell = writer && r >= r0 && r < r1;
         if (h >= k.cutoff && p.e != kDryFlag) {
@@ -880,7 +894,7 @@ __device__ __forceinline__ void adjoint_march_strip(const AdjArgs& a, const int 
             const float Hy = 0.5f * (chi.a + chi.b) - 0.5f * (clo.a + clo.b);
             lhv += fc * LL.b;
             lhu -= fc * LL.c;
-            leta += LL.b * k.g * Hx / k.dx + LL.c * k.g * Hy / k.dy;
+            leta += LL.b * k.g * Hx * inv_dx + LL.c * k.g * Hy * inv_dy;
             if (out_cell && a.wx) {
                 const size_t wo = (size_t)(r - 2) * a.pw + (i - 2);
                 a.wx[wo] = in.wx + LL.b;
@@ -949,10 +963,10 @@ __device__ __forceinline__ void adjoint_march_strip(const AdjArgs& a, const int 
                 const float Rpu = P2.u - __fmul_rn(0.5f, S2.u), Rpv = P2.v - __fmul_rn(0.5f, S2.v);
                 const float fm = flip(EDGE && wallS && jp == 2), fp = flip(EDGE && wallN && jp == ny + 2);
                 const float Hf = 0.5f * (C2.a + C2.b);
-                const float Ep = (P2.e + Hf) - (S2.K - __fmul_rn(k.dy * F2, P2.u * fp)) / k.two_g;
-                const float Em = (P1.e + Hf) + (S1.K - __fmul_rn(k.dy * F1, P1.u * fm)) / k.two_g;
+                const float Ep = (P2.e + Hf) - __fmul_rn(S2.K - __fmul_rn(k.dy * F2, P2.u * fp), inv2g);
+                const float Em = (P1.e + Hf) + __fmul_rn(S1.K - __fmul_rn(k.dy * F1, P1.u * fm), inv2g);
                 const float hp = fmaxf(Ep, 0.0f), hm = fmaxf(Em, 0.0f);
-                const float l0 = (LL2.a - LL1.a) / k.dy, l1 = (LL2.b - LL1.b) / k.dy, l2 = (LL2.c - LL1.c) / k.dy;
+                const float l0 = (LL2.a - LL1.a) * inv_dy, l1 = (LL2.b - LL1.b) * inv_dy, l2 = (LL2.c - LL1.c) * inv_dy;
                 const CuGrad g = cu_vjp(hm, Rmv, Rmu, hp, Rpv, Rpu, l0, l2, l1, k);
                 if (Ep > 0.0f) {
                     A2.a += g.hp;
@@ -981,16 +995,19 @@ __device__ __forceinline__ void adjoint_march_strip(const AdjArgs& a, const int 
                 lL = 0.0f;
             }
             const int bu = (int)(S1.code & 3u), bv = (int)((S1.code >> 2) & 3u), bl = (int)((S1.code >> 4) & 3u);
-            // cells r-1 (A0, pos -1), r (A1, pos 0), r+1 (A2, pos +1)
-            A0.b += B1.a * slope_coef(bu, -1, k.theta) + lL * k.U * pot_coef(bl, -1, k.theta_g, k.half_g) * F0 * uflip_ly(r - 1);
-            A1.b += B1.a * slope_coef(bu, 0, k.theta) + lL * k.U * pot_coef(bl, 0, k.theta_g, k.half_g) * F1 * uflip_ly(r);
-            A2.b += B1.a * slope_coef(bu, 1, k.theta) + lL * k.U * pot_coef(bl, 1, k.theta_g, k.half_g) * F2 * uflip_ly(r + 1);
-            A0.c += B1.b * slope_coef(bv, -1, k.theta);
-            A1.c += B1.b * slope_coef(bv, 0, k.theta);
-            A2.c += B1.b * slope_coef(bv, 1, k.theta);
-            A0.a += lL * k.g * slope_coef(bl, -1, k.theta);
-            A1.a += lL * k.g * slope_coef(bl, 0, k.theta);
-            A2.a += lL * k.g * slope_coef(bl, 1, k.theta);
+            // cells r-1 (A0), r (A1), r+1 (A2)
+            const SlopeAdj au = slope_adj(bu, B1.a, k.theta, 0.5f), av = slope_adj(bv, B1.b, k.theta, 0.5f);
+            const SlopeAdj al = slope_adj(bl, lL, k.theta_g, k.half_g);
+            const float lp = k.U * al.p, lq = k.U * al.q;
+            A0.b += lp * F0 * uflip_ly(r - 1) - au.p;
+            A1.b += (lp + lq) * F1 * uflip_ly(r) + (au.p - au.q);
+            A2.b += lq * F2 * uflip_ly(r + 1) + au.q;
+            A0.c -= av.p;
+            A1.c += av.p - av.q;
+            A2.c += av.q;
+            A0.a -= al.p;
+            A1.a += al.p - al.q;
+            A2.a += al.q;
         }
         // (6) x direction of row j (uniform over the block)
         const bool out_row = j >= r0 && j < r1;
@@ -1003,23 +1020,22 @@ __device__ __forceinline__ void adjoint_march_strip(const AdjArgs& a, const int 
                 const float ul = sb.u[t - 1], uc = P0.u, ur = sb.u[t + 1];
                 const float vl = sb.v[t - 1], vc = P0.v, vr = sb.v[t + 1];
                 const float el = sb.e[t - 1], ec = P0.e, er = sb.e[t + 1];
-                sx.u = minmod_slope(ul, uc, ur, k.theta);
-                sx.v = minmod_slope(vl, vc, vr, k.theta);
-                const int bu = mm_branch((uc - ul) * k.theta, (ur - ul) * 0.5f, (ur - uc) * k.theta);
-                const int bv = mm_branch((vc - vl) * k.theta, (vr - vl) * 0.5f, (vr - vc) * k.theta);
+                int bu, bv;
+                sx.u = mm_slope(ul, uc, ur, k.theta, bu);
+                sx.v = mm_slope(vl, vc, vr, k.theta, bv);
                 const float fvl = (vl * flip(EDGE && ((wallW && i - 1 < 2) || (wallE && i - 1 > nx + 1)))) * F0;
                 const float fvc = (vc * vflip_kx) * F0;
                 const float fvr = (vr * flip(EDGE && ((wallW && i + 1 < 2) || (wallE && i + 1 > nx + 1)))) * F0;
                 const float bw = k.theta_g * ((ec - el) - __fmul_rn(k.V, fvc + fvl));
                 const float ce = k.half_g * ((er - el) - __fmul_rn(k.V, (fvr + __fmul_rn(2.0f, fvc)) + fvl));
                 const float fw = k.theta_g * ((er - ec) - __fmul_rn(k.V, fvc + fvr));
-                const float Kraw = minmod_raw(bw, ce, fw);
                 const int bk = mm_branch(bw, ce, fw);
+                const float Kraw = mm_value(bk, bw, ce, fw);
                 const float dxfv = __fmul_rn(k.dx * F0, vc * vflip_adj);
                 const float Hw = 0.5f * (C0.a + C1.a);
                 const float He = 0.5f * (C0.b + C1.b);
-                const float hw = (ec + Hw) - (Kraw + dxfv) / k.two_g;
-                const float he = (ec + He) + (Kraw + dxfv) / k.two_g;
+                const float hw = (ec + Hw) - __fmul_rn(Kraw + dxfv, inv2g);
+                const float he = (ec + He) + __fmul_rn(Kraw + dxfv, inv2g);
                 float K = Kraw;
                 int ba = kAdjNone;
                 if (!(hw > 0.0f)) { K = -dxfv + __fmul_rn(k.two_g, ec + Hw); ba = kAdjA; }
@@ -1027,7 +1043,7 @@ __device__ __forceinline__ void adjoint_march_strip(const AdjArgs& a, const int 
                 sx.K = K;
                 sx.code = (uint32_t)bu | ((uint32_t)bv << 2) | ((uint32_t)bk << 4) | ((uint32_t)ba << 6) | (1u << 16);
             }
-            sb.su[t] = sx.u; sb.sv[t] = sx.v; sb.sK[t] = sx.K; sb.code[t] = sx.code;
+            sb.su[t] = sx.u; sb.sv[t] = sx.v; sb.sK[t] = sx.K;
             sb.l0[t] = LL0.a; sb.l1[t] = LL0.b; sb.l2[t] = LL0.c;
             __syncthreads();
             // x face (i, i+1)
@@ -1041,12 +1057,12 @@ __device__ __forceinline__ void adjoint_march_strip(const AdjArgs& a, const int 
                 const float Rpv = sb.v[t + 1] - __fmul_rn(0.5f, sb.sv[t + 1]);
                 const float fm = flip(EDGE && wallW && ip == 2), fp = flip(EDGE && wallE && ip == nx + 2);
                 const float Hf = 0.5f * (C0.b + C1.b);
-                const float Ep = (sb.e[t + 1] + Hf) - (sb.sK[t + 1] + __fmul_rn(k.dx * F0, sb.v[t + 1] * fp)) / k.two_g;
-                const float Em = (P0.e + Hf) + (sx.K + __fmul_rn(k.dx * F0, P0.v * fm)) / k.two_g;
+                const float Ep = (sb.e[t + 1] + Hf) - __fmul_rn(sb.sK[t + 1] + __fmul_rn(k.dx * F0, sb.v[t + 1] * fp), inv2g);
+                const float Em = (P0.e + Hf) + __fmul_rn(sx.K + __fmul_rn(k.dx * F0, P0.v * fm), inv2g);
                 const float hp = fmaxf(Ep, 0.0f), hm = fmaxf(Em, 0.0f);
-                const float l0 = (sb.l0[t + 1] - LL0.a) / k.dx;
-                const float l1 = (sb.l1[t + 1] - LL0.b) / k.dx;
-                const float l2 = (sb.l2[t + 1] - LL0.c) / k.dx;
+                const float l0 = (sb.l0[t + 1] - LL0.a) * inv_dx;
+                const float l1 = (sb.l1[t + 1] - LL0.b) * inv_dx;
+                const float l2 = (sb.l2[t + 1] - LL0.c) * inv_dx;
                 const CuGrad g = cu_vjp(hm, Rmu, Rmv, hp, Rpu, Rpv, l0, l1, l2, k);
                 if (Ep > 0.0f) {
                     pe = g.hp;
@@ -1081,22 +1097,18 @@ __device__ __forceinline__ void adjoint_march_strip(const AdjArgs& a, const int 
             } else {
                 lKraw = 0.0f; aux = 0.0f; avx = 0.0f;
             }
-            sb.gu[t] = aux; sb.gv[t] = avx; sb.gK[t] = lKraw;
+            const SlopeAdj gu = slope_adj((int)(sx.code & 3u), aux, k.theta, 0.5f);
+            const SlopeAdj gv = slope_adj((int)((sx.code >> 2) & 3u), avx, k.theta, 0.5f);
+            const SlopeAdj gK = slope_adj((int)((sx.code >> 4) & 3u), lKraw, k.theta_g, k.half_g);
+            sb.gup[t] = gu.p; sb.guq[t] = gu.q; sb.gvp[t] = gv.p; sb.gvq[t] = gv.q; sb.gKp[t] = gK.p; sb.gKq[t] = gK.q;
             __syncthreads();
             // gather the x-slope adjoints of cells i-1, i, i+1
             if (t >= 1 && t < BW - 1) {
-                float lfv = 0.0f;
-                for (int o = -1; o <= 1; ++o) {
-                    const int pos = -o;
-                    const uint32_t c = sb.code[t + o];
-                    if (!(c & (1u << 16))) continue;
-                    A0.b += sb.gu[t + o] * slope_coef((int)(c & 3u), pos, k.theta);
-                    A0.c += sb.gv[t + o] * slope_coef((int)((c >> 2) & 3u), pos, k.theta);
-                    const int bk = (int)((c >> 4) & 3u);
-                    A0.a += sb.gK[t + o] * k.g * slope_coef(bk, pos, k.theta);
-                    lfv -= sb.gK[t + o] * k.V * pot_coef(bk, pos, k.theta_g, k.half_g);
-                }
-                A0.c += lfv * F0 * vflip_kx;
+                const float Kql = sb.gKq[t - 1], Kpr = sb.gKp[t + 1];
+                A0.a += (gK.p - gK.q) + (Kql - Kpr);
+                A0.b += (gu.p - gu.q) + (sb.guq[t - 1] - sb.gup[t + 1]);
+                A0.c += (gv.p - gv.q) + (sb.gvq[t - 1] - sb.gvp[t + 1]) -
+                        k.V * ((gK.p + gK.q) + (Kql + Kpr)) * F0 * vflip_kx;
             }
         }
         // (7) write the adjoint of row j
