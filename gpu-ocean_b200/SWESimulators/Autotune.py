@@ -162,7 +162,7 @@ def tune_batch(batched, candidates=None, graph_lengths=None, steps=20, use_cache
     return result
 
 
-ADJOINT_BATCH_CANDIDATES = [(128, 32), (128, 16), (64, 32), (64, 16)]
+ADJOINT_BATCH_CANDIDATES = [(bw, rows) for bw in (128, 64) for rows in (12, 16, 20, 24, 28, 32)]
 
 
 def tune_adjoint_batch(problem, candidates=None, steps=3):

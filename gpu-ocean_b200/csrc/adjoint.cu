@@ -44,6 +44,9 @@
 // slope gathered by its three cells.  The adjoint of ghost cells is written
 // to the ghost positions and moved to the interior cells they mirror or wrap
 // (k_adj_fold) afterwards.
+#include <math.h>
+
+#include <initializer_list>
 #include <vector>
 
 #include "internal.h"
@@ -1278,34 +1281,65 @@ cudaError_t launch_any(const AdjArgs& a, int kind, cudaStream_t s) {
     return a.land ? launch_form<FRIC, STAGE1, true>(a, kind, s) : launch_form<FRIC, STAGE1, false>(a, kind, s);
 }
 
+// Time (arbitrary units) of `blocks` marching strips of r rows in blocks of bw
+// columns: a strip costs its rows and about 4 more for its priming; whole waves
+// of the resident blocks count in full, the last, partly filled one by a share
+// that grows with its filling, and a row costs less when several waves overlap
+// than when all strips run in step.  The numbers are a fit to heights of 4 .. 64
+// rows on thirteen grids of 400^2 .. 3000^2 and six batches, which picks within
+// 3% of the best of both widths (B200, us per stage adjoint, the rule before /
+// this: 1200^2 139 / 124, 1536^2 244 / 188, 2048^2 296 / 290; us per batched
+// adjoint step, 128 columns x 32 rows before: 8 x 1024^2 1381 / 1357, 16 x 512^2
+// 904 / 817, 4 x 768^2 579 / 484, 32 x 300^2 722 / 662).
+double march_cost(long long blocks, int bw, int r) {
+    const double w = (double)blocks / (148.0 * (512 / bw));
+    const double whole = floor(w), f = w - whole;
+    return (r + 4) * (whole + (f > 0.0 ? 0.5 + 0.5 * f : 0.0)) * (1.0 + 0.4 / ceil(w)) * (bw == 64 ? 1.03 : 1.0);
+}
+
+long long march_blocks(const Scheme& k, int bw, int r) {
+    return (long long)((k.nx + 4 + bw - 7) / (bw - 6)) * ((k.ny + 4 + r - 1) / r);
+}
+
+// Block columns (64 or 128; either where *bw is 0) and rows per strip (where
+// *rows is 0) of least cost for the given grids together.
+template <class Grids>
+void march_shape(const Grids& grids, int* bw, int* rows) {
+    double best = -1.0;
+    const int given_bw = *bw, given_rows = *rows;
+    for (int w = 128; w >= 64; w -= 64) {
+        if (given_bw && w != given_bw) continue;
+        for (int r = 4; r <= 48; r += 4) {
+            if (given_rows) r = given_rows;
+            long long blocks = 0;
+            for (const go_domain* d : grids) blocks += march_blocks(d->k, w, r);
+            const double cost = march_cost(blocks, w, r);
+            if (best < 0.0 || cost < best) { best = cost; *bw = w; *rows = r; }
+            if (given_rows) break;
+        }
+    }
+}
+
 // Launch form and strip (or tile) height for a grid.  A marching block walks
-// its strip sequentially, so below ~300 k cells (512^2) the grid has too few
-// column strips to fill 148 SMs and the tile form is faster (B200: 49.5 vs
-// 58 us per stage at 512^2; 116 vs 170 at 1024^2 the other way).  Marching
-// uses 64-thread blocks up to 1024 columns and 128 above, strips of the power
-// of two in [8, 32] nearest below (column strips x rows) / 600.
+// its strip sequentially, so a small grid has too few strips to fill 148 SMs
+// and the tile form is faster.
 void adjoint_launch(const go_domain* d, int* kind, int* rows) {
     int kd = d->adj_kind;
     const int nx = d->k.nx + 4, ny = d->k.ny + 4;
-    // B200, us per stage adjoint with dependent launches, tiles of 8 / 16 rows
-    // against the 64-column marching form: 512^2 37.5 / 43.4 / 58.0, 640^2
-    // 52.5 / 50.0 / 67.0, 768^2 71.1 / 69.3 / 100.8, 1024^2 (16 rows) 115.0
-    // against 114.4.  The tile form runs up to about 1000^2 cells, with 8-row
-    // tiles (more, smaller CTAs: fewer partial waves) up to about 590^2.
-    // Marching blocks of 64 columns up to 1024 interior columns (1024^2:
-    // 114.4 us against 124 with 128-column blocks).
-    if (kd == GO_ADJ_AUTO) {
-        if ((long long)nx * ny < 1000000LL) kd = GO_ADJ_TILE;
-        else kd = (d->k.nx <= 1024) ? GO_ADJ_MARCH64 : GO_ADJ_MARCH128;
-    }
+    // B200, us per stage adjoint, tiles of 8 / 16 rows against the best
+    // marching strips: 512^2 34.8 / 39.9 / 36.3, 640^2 48.5 / 44.7 / 52.4,
+    // 768^2 65.5 / 61.7 / 67.4, 832^2 (16 rows) 71.8 / 68.5, 896^2 80.1 / 84.6,
+    // 960^2 92.1 / 86.7, 1024^2 104.8 / 87.9.  The tile form runs up to about
+    // 950^2 cells, with 8-row tiles (more, smaller CTAs: fewer partial waves)
+    // up to about 590^2.
+    int bw = kd == GO_ADJ_MARCH64 ? 64 : kd == GO_ADJ_MARCH128 ? 128 : 0;
+    if (kd == GO_ADJ_AUTO && (long long)nx * ny < 900000LL) kd = GO_ADJ_TILE;
     int r = d->adj_rows;
-    if (r <= 0 && kd == GO_ADJ_TILE) {
-        r = ((long long)nx * ny < 350000LL) ? 8 : 16;
-    } else if (r <= 0) {
-        const int bw = (kd == GO_ADJ_MARCH64) ? 64 : 128;
-        const long long target = (long long)((nx + bw - 7) / (bw - 6)) * ny / 600;
-        r = 8;
-        while (r < 32 && 2 * r <= target) r *= 2;
+    if (kd == GO_ADJ_TILE) {
+        if (r <= 0) r = ((long long)nx * ny < 350000LL) ? 8 : 16;
+    } else {
+        march_shape(std::initializer_list<const go_domain*>{d}, &bw, &r);
+        kd = bw == 64 ? GO_ADJ_MARCH64 : GO_ADJ_MARCH128;
     }
     *kind = kd;
     *rows = r;
@@ -1496,6 +1530,8 @@ int go_adjoint_batch_create(go_domain* const* members, int n, go_adjoint_batch**
     b->args.assign(2 * n, AdjArgs());
     b->folds.assign(2 * n, FoldMember());
     b->member_set.assign(n, 0);
+    b->bw = b->rows = 0;
+    march_shape(b->members, &b->bw, &b->rows);
     cudaError_t e = cudaMalloc(&b->d_args, sizeof(AdjArgs) * 2 * n);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_folds, sizeof(FoldMember) * 2 * n);
     if (e != cudaSuccess) {

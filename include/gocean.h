@@ -443,9 +443,10 @@ typedef struct go_state {
  * columns and rows_per_strip = 8, 12 or 16 rows, 0 = automatic: 8 below
  * ~350 k cells, else 16; the forward is recomputed with a 3-cell halo),
  * GO_ADJ_MARCH64 / GO_ADJ_MARCH128 (one thread per column, blocks of 64 or
- * 128 columns marching up strips of rows_per_strip rows, 0 = automatic),
- * GO_ADJ_AUTO (the default: the tile form below ~1 M cells, else marching,
- * 64 up to 1024 columns).  The forms agree to FP32 rounding. */
+ * 128 columns marching up strips of rows_per_strip rows, 0 = the height of
+ * least cost by a fit to measured strips), GO_ADJ_AUTO (the default: the tile
+ * form below 900 k cells, else marching with the width and height of least
+ * cost).  The forms agree to FP32 rounding. */
 #define GO_ADJ_AUTO 0
 #define GO_ADJ_TILE 1
 #define GO_ADJ_MARCH64 2
@@ -490,7 +491,8 @@ int go_adjoint_step(go_domain* d, void* stream, float dt,
 typedef struct go_adjoint_batch go_adjoint_batch;
 int go_adjoint_batch_create(go_domain* const* members, int n, go_adjoint_batch** out);
 int go_adjoint_batch_destroy(go_adjoint_batch* b);
-/* Marching blocks of 64 or 128 columns and strips of rows (0 = 32). */
+/* Marching blocks of 64 or 128 columns and strips of rows (0 = 32).  Default:
+ * the width and height of least cost over all members' strips. */
 int go_adjoint_batch_set_launch(go_adjoint_batch* b, int block_columns, int rows_per_strip);
 int go_adjoint_batch_set_member(go_adjoint_batch* b, int m, float dt,
                                 const go_state* q_n, const go_state* q_star, const go_state* q_next,
