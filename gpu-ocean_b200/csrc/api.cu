@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <string>
 
+#include "cfl.h"
 #include "pair_dispatch.cuh"
 #include "pair_rows.h"
 #include "trace.h"
@@ -204,25 +205,6 @@ __global__ void k_periodic_ew(float* e, float* u, float* v, int p, int nx, int n
     const size_t o = (size_t)j * p + i, s = (size_t)j * p + src;
     e[o] = e[s]; u[o] = u[s]; v[o] = v[s];
 }
-
-// ---------------------------------------------------------------------------
-// CFL limit (max_dt.cu:42-141), exact minimum over all interior cells.
-// ---------------------------------------------------------------------------
-
-__global__ void k_max_dt(const float* eta, const float* hu, const float* hv, int p,
-                         const float* Bm, int pb, int nx, int ny, float dx, float dy, float g,
-                         float land, unsigned int* out) {
-    float best = kRefFltMax;
-    const int n = nx * ny;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
-        const int j = idx / nx + 2, i = idx % nx + 2;
-        const size_t o = (size_t)j * p + i;
-        best = fminf(best, cell_cfl_dt(eta[o], hu[o], hv[o], Bm[(size_t)j * pb + i], dx, dy, g, land, kRefFltMax));
-    }
-    block_min_to(best, out, kRefFltMax);
-}
-
-__global__ void k_fill_u32(unsigned int* p, unsigned int v) { *p = v; }
 
 // ---------------------------------------------------------------------------
 // C ABI
@@ -489,16 +471,8 @@ int go_max_dt(go_domain* d, void* stream, const float* eta, const float* hu, con
     if (!rc) rc = go_check_pitch(Bm_pitch, d->k.nx + 4, "Bm");
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    unsigned int* out = reinterpret_cast<unsigned int*>(dt_dev);
-    unsigned int init_bits;
-    memcpy(&init_bits, &kRefFltMax, sizeof(init_bits));
-    k_fill_u32<<<1, 1, 0, s>>>(out, init_bits);
-    const int n = d->k.nx * d->k.ny;
-    int blocks = (n + 255) / 256;
-    if (blocks > 148 * 8) blocks = 148 * 8;
-    k_max_dt<<<blocks, 256, 0, s>>>(eta, hu, hv, pitch / 4, Bm, Bm_pitch / 4, d->k.nx, d->k.ny, d->k.dx,
-                                     d->k.dy, d->k.g, land_value, out);
-    GO_CUDA(cudaGetLastError());
+    GO_CUDA(cfl_launch(d->k, eta, hu, hv, pitch / 4, Bm, Bm_pitch / 4, land_value, reinterpret_cast<unsigned int*>(dt_dev),
+                       s));
     return GO_OK;
 }
 

@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "cfl.h"
 #include "grf.cuh"
 #include "trace.h"
 #include "pair_dispatch.cuh"
@@ -321,30 +322,6 @@ int batch_launch(go_batch* b, int rk_step, cudaStream_t s, bool follows = false)
     return GO_OK;
 }
 
-// CFL limit of every member in one launch: blockIdx.y is the member, whose
-// current state (h0) is the input of its stage-0 arguments; the cell-mean
-// bathymetry comes from the corners as the set-up computes it.
-__global__ void k_batch_max_dt(const StageArgs* __restrict__ args, unsigned int* __restrict__ out) {
-    const StageArgs& a = args[2 * blockIdx.y];
-    const Scheme& k = a.k;
-    const int n = k.nx * k.ny;
-    float best = kRefFltMax;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
-        const int j = idx / k.nx + 2, i = idx % k.nx + 2;
-        const size_t o = (size_t)j * a.pin + i;
-        const float* H = a.Hi + (size_t)j * a.phi + i;
-        const float Hm = cell_mean_depth(H[0], H[a.phi], H[1], H[a.phi + 1], k.land);
-        best = fminf(best, cell_cfl_dt(a.eta_in[o], a.hu_in[o], a.hv_in[o], Hm, k.dx, k.dy, k.g, k.land,
-                                       kRefFltMax));
-    }
-    block_min_to(best, out + blockIdx.y, kRefFltMax);
-}
-
-__global__ void k_fill_members(unsigned int* p, unsigned int v, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
-}
-
 void drop_graph(go_batch* b) {
     if (b->graph_exec) cudaGraphExecDestroy(b->graph_exec);
     if (b->graph) cudaGraphDestroy(b->graph);
@@ -360,15 +337,9 @@ void drop_graph(go_batch* b) {
 
 // Launches of go_batch_max_dt: every member's CFL limit (float bits) into out.
 int launch_max_dt(go_batch* b, cudaStream_t s, unsigned int* out) {
-    unsigned int init_bits;
-    memcpy(&init_bits, &kRefFltMax, sizeof(init_bits));
-    k_fill_members<<<(b->n + 255) / 256, 256, 0, s>>>(out, init_bits, b->n);
-    long long most = 0;
-    for (const go_domain* d : b->members) most = std::max(most, (long long)d->k.nx * d->k.ny);
-    // about 4 blocks per SM in all, spread over the members
-    const int per_member = (int)std::max(1LL, std::min((most + 255) / 256, (148LL * 4 + b->n - 1) / b->n));
-    k_batch_max_dt<<<dim3(per_member, b->n), 256, 0, s>>>(b->d_args, out);
-    GO_CUDA(cudaGetLastError());
+    int blocks = 1;
+    for (const go_domain* d : b->members) blocks = std::max(blocks, cfl_batch_blocks(d->k, b->n));
+    GO_CUDA(cfl_batch_launch(b->d_args, b->n, blocks, out, s));
     return GO_OK;
 }
 

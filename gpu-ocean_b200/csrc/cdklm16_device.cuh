@@ -161,29 +161,11 @@ __device__ __forceinline__ float cell_mean_depth(float a, float b, float c, floa
     a = dry(a); b = dry(b); c = dry(c); d = dry(d);
     const float wet = 4.0f - (float)(a == kDryFlag) - (float)(b == kDryFlag) - (float)(c == kDryFlag) -
                       (float)(d == kDryFlag);
+    if (wet == 4.0f) return 0.25f * (a + b + c + d);   // the quotient by 4 is exact scaling
     return (wet == 0.0f) ? land : __fdiv_rn(a + b + c + d, wet);   // IEEE quotient, as cell_bm
 }
 
 constexpr float kRefFltMax = 100000.0f;   // max_dt.cu:30 redefines FLT_MAX
-
-// CFL limit of one interior cell (max_dt.cu:42-107): min of 0.25 dx/|u +- c|
-// and 0.25 dy/|v +- c|; `none` for a dry or land cell.  The reference builds
-// max_dt.cu with nvcc's default options (CDKLM16.py:221 passes no compile
-// flags): its quotients and square root are IEEE round-to-nearest, kept here
-// with __fdiv_rn / __fsqrt_rn whatever this library's own flags are.
-__device__ __forceinline__ float cell_cfl_dt(float e, float hu, float hv, float H, float dx, float dy, float g,
-                                             float land, float none) {
-    const float h = e + H;
-    if (h <= 0.0f || fabsf(H - land) < kDryEps) return none;
-    const float u = __fdiv_rn(hu, h);
-    const float v = __fdiv_rn(hv, h);
-    const float c = __fsqrt_rn(g * h);
-    float d = __fdiv_rn(0.25f * dx, fabsf(u + c));
-    d = fminf(d, __fdiv_rn(0.25f * dx, fabsf(u - c)));
-    d = fminf(d, __fdiv_rn(0.25f * dy, fabsf(v + c)));
-    d = fminf(d, __fdiv_rn(0.25f * dy, fabsf(v - c)));
-    return d;
-}
 
 // Block minimum of a positive float, then atomicMin on its bit pattern
 // (positive floats order like their bits).  Every thread of the block calls.

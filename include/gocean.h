@@ -294,13 +294,17 @@ int go_sample_wind(void* stream, const float* field, int w, int h, int nx, int n
 /* Launch shape of the step kernel: shape 0 = 192 threads x 2 blocks/SM,
  * 1 = 192 x 3, 2 = 128 x 4, 3 = 256 x 2, 4 = 128 x 5; 5 = 128 x 5, 6 = 96 x 6
  * and 7 = 192 x 3 with each thread reading its column's inputs two rows
- * ahead through shared memory (cp.async).  Default: when the grid needs more
- * than one wave of blocks, shape 5, or 6 where 96-wide blocks compute at
- * least 4% fewer columns; else 4.  Each block marches down a strip of
- * rows_per_block rows (0 = automatic: the height in {2, 4, 8, 16, 24} that
- * minimises whole waves of blocks times the strip length plus its 4
- * recomputed halo rows).  Chosen by the autotuner; every shape computes
- * identical results. */
+ * ahead through shared memory (cp.async); 8 = the column-pair kernel.  Each
+ * block marches down a strip of rows_per_block rows (0 = automatic: the height
+ * in {2, 4, 8, 16, 24} that minimises whole waves of blocks times the strip
+ * length plus its 4 recomputed halo rows; for shape 8 a multiple of 3 by a fit
+ * to measured heights).  A domain that this call was never made for takes its
+ * kernel from its size: with reciprocal quotients on a north-up grid the tile
+ * kernel (32 x 16 cells per block) below 1.15 million cells, or 350 thousand
+ * where go_domain_set_land told of land; else shape 8 from 1.15 million cells,
+ * or 3500^2 with land; else shape 5, 6 or 4 by the columns they compute.
+ * Chosen by the autotuner among the shapes; every kernel computes identical
+ * results. */
 int go_domain_set_launch(go_domain* d, int shape, int rows_per_block);
 /* Shape 8: the column-pair kernel.  Blocks of 64 threads, each thread two
  * adjacent columns in packed FP32x2 arithmetic (sm_100 FADD2/FFMA2), inputs
@@ -400,8 +404,10 @@ int go_batch_set_member(go_batch* b, int m, float dt, float* eta0, float* hu0, f
 
 /* Launch shape (as go_domain_set_launch) and persistent grid size: blocks
  * = 0 launches one block per tile, blocks > 0 that many blocks walking the
- * tile list.  Default: 32-row strips, one block per tile, and the shape
- * chosen as for a single grid from the column work of all members. */
+ * tile list.  A batch that this call was never made for takes the tile kernel
+ * for narrow members and otherwise shape 8 with the strip height that suits
+ * all members' strips, or 4 with few cells in all, one block per tile; shape 4
+ * with 16-row strips where a member was told that it may have land. */
 int go_batch_set_launch(go_batch* b, int shape, int rows_per_block, int blocks);
 int go_batch_set_arith(go_batch* b, int mode);
 
