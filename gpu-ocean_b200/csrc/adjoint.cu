@@ -1494,6 +1494,9 @@ int adjoint_batch_commit(go_adjoint_batch* b) {
     GO_CUDA(cudaMemcpy(b->d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice));
     GO_CUDA(cudaMemcpy(b->d_args, b->args.data(), sizeof(AdjArgs) * b->args.size(), cudaMemcpyHostToDevice));
     GO_CUDA(cudaMemcpy(b->d_folds, b->folds.data(), sizeof(FoldMember) * b->folds.size(), cudaMemcpyHostToDevice));
+    // the copies may return before their transfers have ended, and the batch's
+    // stream does not wait for the default stream
+    GO_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     b->dirty = false;
     return GO_OK;
 }

@@ -32,6 +32,7 @@ struct EventLoop {
     uint32_t event;      // model-error event of the current event
     int events_left;
     long long steps;
+    int stalled;         // the time step cannot end the event: both loops stop
 };
 
 // What a captured event-loop graph depends on besides the loop state.
@@ -229,8 +230,7 @@ int batch_commit_tile(go_batch* b) {
     return GO_OK;
 }
 
-int batch_commit(go_batch* b) {
-    if (!b->dirty) return GO_OK;
+int batch_lay_out(go_batch* b) {
     for (int m = 0; m < b->n; ++m)
         if (!b->member_set[m]) return go_fail(GO_ERR_INVALID, "batch member %d has no state set", m);
     int rc = batch_variant(b);
@@ -261,6 +261,16 @@ int batch_commit(go_batch* b) {
     b->ntiles = (int)tiles.size();
     b->dirty = false;
     return GO_OK;
+}
+
+// The lists and arguments on the device.  A copy from pageable memory may
+// return before its transfer has ended, and the callers' streams do not wait
+// for the default stream: waited for here.
+int batch_commit(go_batch* b) {
+    if (!b->dirty) return GO_OK;
+    const int rc = batch_lay_out(b);
+    if (!rc) GO_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    return rc;
 }
 
 int batch_launch_pair(go_batch* b, int rk_step, cudaStream_t s) {
@@ -374,6 +384,11 @@ int grf_prepare(go_batch* b, const GrfWeights& W) {
 }
 
 // ---- device-driven event loop ----------------------------------------------
+// More steps than any event takes: a time step of zero (the CFL limit of an
+// infinite speed), or one of which an event would take more than this, ends the
+// device's loops, which the host then reports.
+constexpr double kMaxEventSteps = 1.0e7;
+
 // The step of the event that starts at t_now: the common dt, or the model
 // time left in the event rounded to float32 when that is shorter, which
 // makes it the event's last step (CDKLM16.py:508-517: local_dt =
@@ -382,6 +397,7 @@ int grf_prepare(go_batch* b, const GrfWeights& W) {
 __device__ __forceinline__ float event_step_dt(EventLoop* L) {
     const float rem = __double2float_rn(__dsub_rn(L->interval, L->t_now));
     const float local = fminf(L->dt, rem);
+    if ((double)L->dt * kMaxEventSteps < L->interval) L->last = L->stalled = 1;
     if (local != L->dt) L->last = 1;
     return local;
 }
@@ -448,7 +464,7 @@ __global__ void k_event_end(EventLoop* L, const unsigned int* __restrict__ cfl, 
         L->dt = dt;
         L->event += 1;
         L->events_left -= 1;
-        cudaGraphSetConditional(events, L->events_left > 0 ? 1u : 0u);
+        cudaGraphSetConditional(events, L->events_left > 0 && !L->stalled ? 1u : 0u);
         red[0] = dt;
     }
     __syncthreads();
@@ -900,6 +916,9 @@ int go_batch_run_events(go_batch* b, void* stream, uint32_t first_event, int n_e
     }
     if (steps_out) *steps_out = L.steps;
     if (dt_out) *dt_out = L.dt;
+    if (L.stalled)
+        return go_fail(GO_ERR_INVALID, "event %u: its time step is zero or too short to end an event of %g s", L.event - 1,
+                       interval);
     return GO_OK;
 }
 
