@@ -42,13 +42,15 @@ int go_check_pitch(int pitch_bytes, int min_floats, const char* what) {
 // in.  The numbers are a fit to heights of 9 .. 120 rows on ten grids of 1280^2 ..
 // 4096^2 (B200, us per RK2 step, one simulator and three on their own streams;
 // the height taken / others): 1280^2 12 rows 87 and 61 / 18 97 and 60, 2048^2 30
-// rows 177 and 134 / 24 209 and 136, 3072^2 66 rows 350 and 285 / 36 373 and 289,
-// 4096^2 60 rows 597 and 513 / 24 585 and 528, 42 611 and 517.
+// rows 177 and 134 / 24 209 and 136, 3072^2 33 rows 348 and 289 / 36 373 and 289,
+// 4096^2 30 rows 585 and 522 / 24 585 and 528, 42 611 and 517.  Strips above 36 rows
+// are left out: three simulators gain 1 to 2% with them, one alone loses as much
+// (4096^2 60 rows 597 and 513).
 static int pair_rows(int nx, int ny) {
     const long long strips = go::shape_columns(GO_SHAPE_PAIR, nx) / go::shape_block_width(GO_SHAPE_PAIR);
     int best = 3;
     double best_cost = -1.0;
-    for (int r = 3; r <= 120; r += 3) {
+    for (int r = 3; r <= 36; r += 3) {
         const double cost = go::pair_strip_cost(strips * ((std::max(ny - 4, 1) + r - 1) / r), r) * (1.0 + 1.5 / r);
         if (best_cost < 0.0 || cost < best_cost) { best = r; best_cost = cost; }
     }
