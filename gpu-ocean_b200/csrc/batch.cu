@@ -354,8 +354,12 @@ int launch_max_dt(go_batch* b, cudaStream_t s, unsigned int* out) {
 }
 
 // Model-error descriptors of the members (their eta buffers, sizes,
-// boundary kinds, member keys, scratch offsets) for filter radius W.R.
-int grf_prepare(go_batch* b, const GrfWeights& W) {
+// boundary kinds, member keys, scratch offsets) for filter radius W.R.  Their
+// upload is ordered on s, after the filters queued there that read the
+// descriptors before and ahead of the next (a copy on the default stream is
+// neither: s does not wait for it, nor it for s), and waited for, since it
+// reads a host array that ends with this call.
+int grf_prepare(go_batch* b, const GrfWeights& W, cudaStream_t s) {
     if (b->d_grf && b->grf_R == W.R) return GO_OK;
     std::vector<GrfMember> h(b->n);
     size_t off = 0;
@@ -375,7 +379,8 @@ int grf_prepare(go_batch* b, const GrfWeights& W) {
         my = max(my, k.ny);
     }
     if (!b->d_grf) GO_CUDA(cudaMalloc(&b->d_grf, sizeof(GrfMember) * b->n));
-    GO_CUDA(cudaMemcpy(b->d_grf, h.data(), sizeof(GrfMember) * b->n, cudaMemcpyHostToDevice));
+    GO_CUDA(cudaMemcpyAsync(b->d_grf, h.data(), sizeof(GrfMember) * b->n, cudaMemcpyHostToDevice, s));
+    GO_CUDA(cudaStreamSynchronize(s));
     b->grf_R = W.R;
     b->grf_scratch = off;
     b->grf_max_nx = mx;
@@ -841,7 +846,7 @@ int go_batch_grf_perturb(go_batch* b, void* stream, uint32_t key0, uint32_t even
     rc = grf_weights(corr_cells, &W);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    rc = grf_prepare(b, W);
+    rc = grf_prepare(b, W, s);
     if (rc) return rc;
     if (scratch_floats < b->grf_scratch)
         return go_fail(GO_ERR_INVALID, "scratch holds %zu floats, the batch needs %zu", scratch_floats,
@@ -865,7 +870,7 @@ int go_batch_run_events(go_batch* b, void* stream, uint32_t first_event, int n_e
     GrfWeights W;
     rc = grf_weights(corr_cells, &W);
     if (rc) return rc;
-    rc = grf_prepare(b, W);
+    rc = grf_prepare(b, W, s);
     if (rc) return rc;
     if (scratch_floats < b->grf_scratch)
         return go_fail(GO_ERR_INVALID, "scratch holds %zu floats, the batch needs %zu", scratch_floats,

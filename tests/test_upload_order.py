@@ -1,0 +1,64 @@
+"""Uploads and clears of device memory by the native library: what a caller's
+stream reads next is in place before it can be read.
+
+A copy from pageable host memory, or a cudaMemset, on the default stream may
+still be under way when its call returns, and the callers' (non-blocking)
+streams do not wait for that stream; nor does it wait for kernels queued on
+theirs that still read what is overwritten."""
+
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gpu-ocean_b200", "csrc")
+
+
+def _function(source, name):
+    """Text of the function `name` of a source file: from its definition to the
+    closing brace in the first column (or the indentation of its first line)."""
+    text = open(os.path.join(CSRC, source)).read()
+    m = re.search(r"^[\w:<>&* \t\"]*\b%s\([^;{]*\{$" % name, text, re.M)
+    assert m, name
+    return text[m.start():text.index("\n}\n", m.end())]
+
+
+def test_model_error_descriptors_are_uploaded_on_the_callers_stream():
+    body = _function("batch.cu", "grf_prepare")
+    assert "cudaMemcpy(" not in body
+    copy, wait = body.index("cudaMemcpyAsync(b->d_grf"), body.index("cudaStreamSynchronize(s)")
+    assert re.search(r"cudaMemcpyAsync\(b->d_grf[^;]*, s\)", body) and copy < wait
+
+
+@pytest.mark.gpu
+def test_model_error_with_another_correlation_length_waits_for_the_filter_before():
+    """Two perturbations of different correlation lengths queued behind work on
+    the batch's stream: each filter reads its own descriptors, so the states
+    are those of the same perturbations one at a time."""
+    import numpy as np
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    from SWESimulators import BatchedEnsemble, CDKLM16, Common
+    ctx = Common.CUDAContext()
+
+    def ensemble():
+        sims = []
+        for nx, ny in ((130, 96), (64, 200), (96, 33)):
+            zero = np.zeros((ny + 4, nx + 4), np.float32)
+            H = np.full((ny + 5, nx + 5), 50.0, np.float32)
+            sims.append(CDKLM16.CDKLM16(ctx, zero, zero, zero, H, nx, ny, 1000.0, 1000.0, 1.0, 9.81, 1.2e-4, 0.0, 0.0))
+        return BatchedEnsemble.BatchedCDKLM16(sims)
+    got, want = ensemble(), ensemble()
+    got.model_error(1, corr_cells=4.0)               # the batch's lists and the scratch are laid out
+    torch.cuda.synchronize()
+    with torch.cuda.stream(got.stream):
+        torch.cuda._sleep(40_000_000)                # some 20 ms at the SM clock
+    for event, corr in ((2, 15.0), (3, 4.0), (4, 15.0)):
+        got.model_error(event, corr_cells=corr)
+    for event, corr in ((1, 4.0), (2, 15.0), (3, 4.0), (4, 15.0)):
+        want.model_error(event, corr_cells=corr)
+        torch.cuda.synchronize()
+    torch.cuda.synchronize()
+    for a, b in zip(got.sims, want.sims):
+        assert np.array_equal(a.download()[0], b.download()[0])
