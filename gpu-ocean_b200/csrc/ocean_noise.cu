@@ -897,6 +897,9 @@ int go_noise_batch_create(const go_noise_member* members, int n, int nx, int ny,
     if (!rc) e = cudaMalloc(&b->d_members, sizeof(go_noise_member) * n);
     if (!rc && e == cudaSuccess)
         e = cudaMemcpy(b->d_members, members, sizeof(go_noise_member) * n, cudaMemcpyHostToDevice);
+    // the copy may return before its transfer has ended, and the stream of the
+    // first perturbation does not wait for the default stream
+    if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (rc || e != cudaSuccess) {
         if (b->d_members) cudaFree(b->d_members);
         delete b;

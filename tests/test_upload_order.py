@@ -30,6 +30,17 @@ def test_model_error_descriptors_are_uploaded_on_the_callers_stream():
     assert re.search(r"cudaMemcpyAsync\(b->d_grf[^;]*, s\)", body) and copy < wait
 
 
+# functions that fill device memory through the default stream, and the last
+# such call of each: it is followed by a wait for that stream
+WAITED = [("ocean_noise.cu", "go_noise_batch_create", "cudaMemcpy(b->d_members")]
+
+
+@pytest.mark.parametrize("source,name,last", WAITED, ids=[w[1] for w in WAITED])
+def test_uploads_on_the_default_stream_are_waited_for(source, name, last):
+    body = _function(source, name)
+    assert "cudaStreamSynchronize(cudaStreamLegacy)" in body[body.rindex(last):]
+
+
 @pytest.mark.gpu
 def test_model_error_with_another_correlation_length_waits_for_the_filter_before():
     """Two perturbations of different correlation lengths queued behind work on
