@@ -5,6 +5,7 @@
 // --ftz=true --prec-div=false --prec-sqrt=false --fmad=false.
 #include <algorithm>
 #include <string>
+#include <vector>
 
 #include "cfl.h"
 #include "pair_dispatch.cuh"
@@ -265,6 +266,9 @@ int go_domain_create(const go_domain_desc* desc, go_domain** out) {
     if (e == cudaSuccess) e = cudaMemset(d->d_frows, 0, sizeof(float) * (s.ny + 4));
     if (e == cudaSuccess) e = cudaMalloc(&d->d_status, sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMemset(d->d_status, 0, sizeof(unsigned int));
+    // a memset may return before it has run, and the steps' streams do not
+    // wait for the default stream
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e != cudaSuccess) {
         cudaFree(d->d_frows);
         cudaFree(d->d_status);
@@ -294,16 +298,16 @@ int go_domain_destroy(go_domain* d) {
 int go_domain_set_coriolis(go_domain* d, const float* f_rows_host, int n) {
     if (!d || !f_rows_host) return go_fail(GO_ERR_INVALID, "null argument");
     const int rows = d->k.ny + 4;
+    if (n != 1 && n != rows)
+        return go_fail(GO_ERR_INVALID, "Coriolis table has %d rows, need 1 or ny+4 = %d", n, rows);
+    std::vector<float> plane;
     if (n == 1) {
-        float* tmp = new float[rows];
-        for (int j = 0; j < rows; ++j) tmp[j] = f_rows_host[0];
-        cudaError_t e = cudaMemcpy(d->d_frows, tmp, sizeof(float) * rows, cudaMemcpyHostToDevice);
-        delete[] tmp;
-        GO_CUDA(e);
-        return GO_OK;
+        plane.assign(rows, f_rows_host[0]);
+        f_rows_host = plane.data();
     }
-    if (n != rows) return go_fail(GO_ERR_INVALID, "Coriolis table has %d rows, need 1 or ny+4 = %d", n, rows);
     GO_CUDA(cudaMemcpy(d->d_frows, f_rows_host, sizeof(float) * rows, cudaMemcpyHostToDevice));
+    // the copy may return before its transfer has ended
+    GO_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     return GO_OK;
 }
 
@@ -483,7 +487,11 @@ int go_domain_status(go_domain* d, uint32_t* status, int clear) {
     unsigned int v = 0;
     GO_CUDA(cudaMemcpy(&v, d->d_status, sizeof(v), cudaMemcpyDeviceToHost));
     *status = v;
-    if (clear) GO_CUDA(cudaMemset(d->d_status, 0, sizeof(unsigned int)));
+    if (clear) {
+        GO_CUDA(cudaMemset(d->d_status, 0, sizeof(unsigned int)));
+        // a bit that a later step sets is not lost to a clear still under way
+        GO_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    }
     return GO_OK;
 }
 

@@ -84,7 +84,7 @@ int go_domain_destroy(go_domain* d);
 /* Coriolis parameter per ghost-inclusive row j = 0..ny+3, as the reference
  * samples its f texture at cell centres (CDKLM16_kernel.cu:49-58;
  * texture built at CDKLM16.py:310-351).  n == 1 sets an f-plane.
- * Synchronous host->device copy. */
+ * Synchronous host->device copy; not while a step of the domain is in flight. */
 int go_domain_set_coriolis(go_domain* d, const float* f_rows_host, int n);
 
 /* Uniform wind stress (kinematic, N/m^2 / rho_w): current and next values

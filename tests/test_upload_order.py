@@ -32,7 +32,10 @@ def test_model_error_descriptors_are_uploaded_on_the_callers_stream():
 
 # functions that fill device memory through the default stream, and the last
 # such call of each: it is followed by a wait for that stream
-WAITED = [("ocean_noise.cu", "go_noise_batch_create", "cudaMemcpy(b->d_members")]
+WAITED = [("ocean_noise.cu", "go_noise_batch_create", "cudaMemcpy(b->d_members"),
+          ("api.cu", "go_domain_create", "cudaMemset(d->d_status"),
+          ("api.cu", "go_domain_set_coriolis", "cudaMemcpy(d->d_frows"),
+          ("api.cu", "go_domain_status", "cudaMemset(d->d_status")]
 
 
 @pytest.mark.parametrize("source,name,last", WAITED, ids=[w[1] for w in WAITED])
