@@ -151,6 +151,9 @@ int go_wind_texture_create(const float* field, int w, int h, uint64_t* texture) 
     GO_CUDA(cudaMallocArray(&arr, &ch, w, h));
     cudaError_t e = cudaMemcpy2DToArray(arr, 0, 0, field, sizeof(float) * w, sizeof(float) * w, h,
                                         cudaMemcpyHostToDevice);
+    // the copy may return before its transfer has ended, and the streams that
+    // sample the texture do not wait for the default stream
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     cudaTextureObject_t tex = 0;
     if (e == cudaSuccess) {
         cudaResourceDesc res;

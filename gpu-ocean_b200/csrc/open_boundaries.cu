@@ -182,6 +182,9 @@ int go_bc_texture_create(const float* texels, int w, int h, uint64_t* texture) {
     GO_CUDA(cudaMallocArray(&arr, &ch, w, h));
     cudaError_t e = cudaMemcpy2DToArray(arr, 0, 0, texels, sizeof(float4) * w, sizeof(float4) * w, h,
                                         cudaMemcpyHostToDevice);
+    // the copy may return before its transfer has ended, and the streams that
+    // sample the texture do not wait for the default stream
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     cudaTextureObject_t tex = 0;
     if (e == cudaSuccess) {
         cudaResourceDesc res;

@@ -35,7 +35,24 @@ def test_model_error_descriptors_are_uploaded_on_the_callers_stream():
 WAITED = [("ocean_noise.cu", "go_noise_batch_create", "cudaMemcpy(b->d_members"),
           ("api.cu", "go_domain_create", "cudaMemset(d->d_status"),
           ("api.cu", "go_domain_set_coriolis", "cudaMemcpy(d->d_frows"),
-          ("api.cu", "go_domain_status", "cudaMemset(d->d_status")]
+          ("api.cu", "go_domain_status", "cudaMemset(d->d_status"),
+          ("drifters.cu", "go_wind_texture_create", "cudaMemcpy2DToArray("),
+          ("open_boundaries.cu", "go_bc_texture_create", "cudaMemcpy2DToArray("),
+          ("batch.cu", "batch_commit", "batch_lay_out("),     # calls all that fills the batch's lists
+          ("adjoint.cu", "adjoint_batch_commit", "cudaMemcpy(b->d_folds")]
+
+
+def test_every_upload_is_listed():
+    """No other function uses the default stream to fill device memory."""
+    layouts = ("batch_commit_pair", "batch_commit_tile", "batch_lay_out", "tile_batch_consts")   # within batch_commit
+    known = {w[1] for w in WAITED} | set(layouts)
+    for source in sorted(os.listdir(CSRC)):
+        text = open(os.path.join(CSRC, source)).read()
+        for m in re.finditer(r"\b(cudaMemcpy|cudaMemset|cudaMemcpy2D|cudaMemcpyToSymbol|cudaMemcpy2DToArray)\(([^;]*);", text):
+            if "DeviceToHost" in m.group(2) or "//" in text[text.rindex("\n", 0, m.start()):m.start()]:
+                continue
+            head = re.findall(r"^[\w:<>&*\" ]+?(\w+)\([^;{]*\{$", text[:m.start()], re.M)
+            assert head[-1] in known, (source, head[-1])
 
 
 @pytest.mark.parametrize("source,name,last", WAITED, ids=[w[1] for w in WAITED])
