@@ -321,7 +321,11 @@ class BatchedCDKLM16:
         must share dt (update_dt), carry no OceanStateNoise model error of
         their own and no time-varying wind.  Otherwise, or with
         device_loop=False, the host drives each event (one CFL read-back per
-        event); both give the same states, times and steps bit for bit."""
+        event); both give the same states, times and steps bit for bit.
+
+        An event whose time step is zero or far too short to end it is not
+        begun and raises; the members' states, t, num_iterations and dt are
+        then those after the events before it."""
         dts = {float(np.float32(s.dt)) for s in self.sims}
         if device_loop and len(dts) == 1 and not self._time_varying_wind() and not self._has_model_error():
             return self._run_events_device(first_event, n_events, interval, std, corr_cells, courant)
@@ -357,14 +361,21 @@ class BatchedCDKLM16:
             buf = torch.empty(int(n), dtype=torch.float32, device="cuda")
             self._loop_scratch = buf
         t0 = [float(s.t) for s in self.sims]
-        t, steps, dt = self.batch.run_events(self.stream, first_event, n_events, float(interval),
-                                             np.float32(self.sims[0].dt), float(courant),
-                                             ModelError.MODEL_ERROR_SEED, float(std), float(corr_cells), buf, t0)
+        failed = None
+        try:
+            after = self.batch.run_events(self.stream, first_event, n_events, float(interval),
+                                          np.float32(self.sims[0].dt), float(courant), ModelError.MODEL_ERROR_SEED,
+                                          float(std), float(corr_cells), buf, t0)
+        except _native.NativeError as err:
+            failed, after = err, err.progress       # the events before the one that was not begun
+        t, steps, dt = after
         for s, tm in zip(self.sims, t):
             s.t = float(tm)
             s.num_iterations += steps
             s.dt = dt
         self._release_members()
+        if failed is not None:
+            raise failed
         return steps
 
     def synchronize(self):

@@ -374,14 +374,22 @@ class Batch:
 
     def run_events(self, stream, first_event, n_events, interval, dt, courant, key0, std, corr_cells, scratch, t):
         """go_batch_run_events; t: the members' model times (float64, member
-        order).  Returns (t after, steps per member, common dt after)."""
+        order).  Returns (t after, steps per member, common dt after); a
+        NativeError carries them as its ``progress`` (an event that is not
+        begun leaves the states after the events before it)."""
         tt = np.ascontiguousarray(np.asarray(t, dtype=np.float64).reshape(-1))
         assert tt.size == self.n
         steps = ctypes.c_longlong()
-        dt_out = ctypes.c_float()
-        check(load().go_batch_run_events(self.handle, stream_handle(stream), int(first_event) & 0xFFFFFFFF,
-                                         int(n_events), float(interval), float(np.float32(dt)), float(courant),
-                                         int(key0) & 0xFFFFFFFF, float(std), float(corr_cells), ptr(scratch),
-                                         int(scratch.numel()), tt.ctypes.data_as(ctypes.c_void_p),
-                                         ctypes.byref(steps), ctypes.byref(dt_out)))
-        return tt, int(steps.value), np.float32(dt_out.value)
+        dt_out = ctypes.c_float(float(np.float32(dt)))
+        rc = load().go_batch_run_events(self.handle, stream_handle(stream), int(first_event) & 0xFFFFFFFF,
+                                        int(n_events), float(interval), float(np.float32(dt)), float(courant),
+                                        int(key0) & 0xFFFFFFFF, float(std), float(corr_cells), ptr(scratch),
+                                        int(scratch.numel()), tt.ctypes.data_as(ctypes.c_void_p),
+                                        ctypes.byref(steps), ctypes.byref(dt_out))
+        after = tt, int(steps.value), np.float32(dt_out.value)
+        try:
+            check(rc)
+        except NativeError as err:
+            err.progress = after
+            raise
+        return after

@@ -604,7 +604,11 @@ int go_batch_grf_perturb(go_batch* b, void* stream, uint32_t key0, uint32_t even
  * captured on the first call and reused while key0, std_dev, corr_cells,
  * scratch and the batch's members and launch stay the same; scratch must
  * stay allocated while it is in use.  Wind stays at the members' bound
- * wind_stress_t.  Synchronous. */
+ * wind_stress_t.  Synchronous.
+ *
+ * An event whose time step is zero, or of which it would take more than 5e8,
+ * is not begun: GO_ERR_INVALID, with the states, t_members, steps_out and dt_out
+ * (the step that is too short, now every member's) those after the events before. */
 int go_batch_run_events(go_batch* b, void* stream, uint32_t first_event, int n_events,
                         double interval, float dt, double courant, uint32_t key0,
                         float std_dev, float corr_cells, float* scratch,
