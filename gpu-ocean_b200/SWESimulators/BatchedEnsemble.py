@@ -177,6 +177,8 @@ class BatchedCDKLM16:
             local_dt = np.float32(min(dt, np.float32(t_end - t_now)))
             if local_dt != dt:
                 break
+            if t_now + np.float64(local_dt) <= t_now:
+                raise ValueError("a time step of %g s does not advance the model time" % local_dt)
             full += 1
             t_now += np.float64(local_dt)
         if full and perturb:

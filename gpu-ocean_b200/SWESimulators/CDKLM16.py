@@ -251,6 +251,10 @@ class CDKLM16(Simulator.Simulator):
                     pending_n = 0
                 self.updateDt()
             local_dt = np.float32(min(self.dt, np.float32(t_end - t_now)))
+            if t_now + np.float64(local_dt) <= t_now:
+                if pending_n:
+                    self._launch_steps(pending_n, pending_dt, pending_w)
+                raise ValueError("a time step of %g s does not advance the model time" % local_dt)
             wind_t = np.float32(self.update_wind_stress())
             if pending_n and (local_dt != pending_dt or wind_t != pending_w or one_by_one):
                 self._launch_steps(pending_n, pending_dt, pending_w)
@@ -284,9 +288,10 @@ class CDKLM16(Simulator.Simulator):
         step loop takes next: while float32(min(self.dt, float32(t_end -
         t_now))) is dt, with t_now and self.t advancing by float64(dt) each
         step, in the loop's own float64 sums.  The time left is compared in
-        float64 and rounded as the loop does only when it is near dt."""
+        float64 and rounded as the loop does only when it is near dt.  None
+        for a dt that may not advance the sum, which the loop checks."""
         step, limit = float(dt), float(self.dt)
-        if np.float32(limit) != dt:
+        if np.float32(limit) != dt or float(t_end) + step <= float(t_end):
             return 0, t_now
         t, now, end, n = float(self.t), float(t_now), float(t_end), 0
         near = max(step, limit) * (1.0 + 1.0e-6)
