@@ -27,6 +27,7 @@ GO_STATUS_ADJ_SCOPE = 0x2
 GO_STATUS_TIMEOUT = 0x4
 GO_STATUS_BOUNDS = 0x8
 GO_DEBUG_SKIP_TMA = 0x1
+GO_DEBUG_STEPS_ANY_SIZE = 0x2
 GO_ERR_INVALID = -1
 GO_ERR_CUDA = -2
 GO_ERR_UNSUPPORTED = -3

@@ -449,8 +449,11 @@ int go_cdklm_step(go_domain* d, void* stream, int n_steps, float dt, float wind_
     const StageArgs a1 = go_stage_args(d, dt, 1, eta1, hu1, hv1, pitch1 / 4, eta0, hu0, hv0, pitch0 / 4, Hi,
                                        Hi_pitch / 4, land_value, wind_stress_t);
     const bool open = go_has_open_bc(d);
-    if (!open && go_tile_stage(d, a0) && go_tile_stage(d, a1) && go_tile_steps_fit(d))
-        return go_launch_tile_steps(d, s, a0, n_steps);
+    if (!open && go_tile_stage(d, a0) && go_tile_stage(d, a1) && go_tile_steps_fit(d)) {
+        bool done = false;
+        rc = go_launch_tile_steps(d, s, a0, n_steps, &done);
+        if (rc || done) return rc;
+    }
     PreparedStage p0, p1;
     rc = go_prepare_stage(d, a0, &p0);
     if (!rc) rc = go_prepare_stage(d, a1, &p1);
@@ -497,7 +500,7 @@ int go_domain_status(go_domain* d, uint32_t* status, int clear) {
 
 int go_domain_set_debug(go_domain* d, unsigned flags) {
     if (!d) return go_fail(GO_ERR_INVALID, "null domain");
-    if (flags & ~GO_DEBUG_SKIP_TMA) return go_fail(GO_ERR_INVALID, "unknown debug flags 0x%x", flags);
+    if (flags & ~(GO_DEBUG_SKIP_TMA | GO_DEBUG_STEPS_ANY_SIZE)) return go_fail(GO_ERR_INVALID, "unknown debug flags 0x%x", flags);
     d->debug = flags;
     return GO_OK;
 }

@@ -315,8 +315,8 @@ int batch_launch_pair(go_batch* b, int rk_step, cudaStream_t s) {
 // follows: the launch before it on the stream is a stage of the same call.
 int batch_launch(go_batch* b, int rk_step, cudaStream_t s, bool follows = false) {
     if (b->tile) {
-        const cudaError_t e = tile_batch_launch(TileBatchReq{b->d_args, b->d_dt, b->d_tile_consts, b->d_tiles, b->ntiles,
-                                                             rk_step, b->members[0]->device, s, follows});
+        const cudaError_t e = tile_batch_launch(
+            TileBatchReq{b->d_args, b->d_dt, b->d_tile_consts, b->d_tiles, b->ntiles, rk_step, s, follows});
         if (e != cudaSuccess) return go_fail(GO_ERR_CUDA, "batch stage launch (tiles) failed: %s", cudaGetErrorString(e));
         return GO_OK;
     }

@@ -87,7 +87,7 @@ int go_tile_setup(go_domain* d);
 bool go_tile_stage(const go_domain* d, const go::StageArgs& a);
 int go_launch_tile(go_domain* d, cudaStream_t s, const go::StageArgs& a, bool follows);
 bool go_tile_steps_fit(const go_domain* d);
-int go_launch_tile_steps(go_domain* d, cudaStream_t s, const go::StageArgs& a, int n);
+int go_launch_tile_steps(go_domain* d, cudaStream_t s, const go::StageArgs& a, int n, bool* done);
 
 // Column-pair shape (pair_launch.cu).
 bool go_pair_shape(int shape);

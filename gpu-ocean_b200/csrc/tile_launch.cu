@@ -1,5 +1,6 @@
 // Launches of the tile stage kernels (cdklm16_tile.cuh).
-#include <atomic>
+#include <limits.h>
+
 #include <vector>
 
 #include "cdklm16_tile.cuh"
@@ -14,19 +15,12 @@ constexpr long long kTileCells = 1150LL * 1000LL, kTileLandCells = 350LL * 1000L
 
 dim3 tile_grid(const Scheme& k) { return dim3((k.nx + kTileX - 1) / kTileX, (k.ny + kTileY - 1) / kTileY); }
 
-// The kernels' shared-memory size, allowed once per device.
-cudaError_t allow_smem(int device) {
-    static std::atomic<unsigned long long> done{0};
-    const unsigned long long bit = 1ULL << (device & 63);
-    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
-    const int bytes = (int)sizeof(TileSmem);
-    cudaError_t e = cudaFuncSetAttribute(cdklm_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(cdklm_tile_steps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(cdklm_tile_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
-    return e;
+// Allows a kernel its shared-memory size in the current context.  Done for
+// each domain and batch layout, whose device memory belongs to that context
+// too, and not once per process, which a reset of the device would undo.
+template <class K>
+cudaError_t allow_smem(K kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem));
 }
 
 // 32-bit byte offsets into every array of a stage.
@@ -52,10 +46,14 @@ cudaLaunchConfig_t tile_config(dim3 grid, cudaStream_t s, cudaLaunchAttribute* a
 
 int go_tile_setup(go_domain* d) {
     if ((long long)d->k.nx * d->k.ny >= kTileCells) return GO_OK;
-    int sms = 0, coop = 0;
+    GO_CUDA(allow_smem(cdklm_tile_kernel));
+    GO_CUDA(allow_smem(cdklm_tile_steps_kernel));
+    int sms = 0, coop = 0, per_sm = 0;
     GO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device));
     GO_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, d->device));
-    d->tile_steps_blocks = coop ? sms : 0;
+    GO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cdklm_tile_steps_kernel, kTileThreads,
+                                                          sizeof(TileSmem)));
+    d->tile_steps_blocks = coop && per_sm > 0 ? sms : 0;
     return GO_OK;
 }
 
@@ -81,8 +79,7 @@ int go_launch_tile(go_domain* d, cudaStream_t s, const StageArgs& a, bool follow
     cudaLaunchAttribute attr;
     const cudaLaunchConfig_t cfg = tile_config(tile_grid(a.k), s, &attr, follows);
     d->stage_launches = 1;
-    cudaError_t e = allow_smem(d->device);
-    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, cdklm_tile_kernel, a, tile_const(a.k));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, cdklm_tile_kernel, a, tile_const(a.k));
     if (e != cudaSuccess) return go_fail(GO_ERR_CUDA, "stage launch (tile) failed: %s", cudaGetErrorString(e));
     return GO_OK;
 }
@@ -95,19 +92,27 @@ int go_launch_tile(go_domain* d, cudaStream_t s, const StageArgs& a, bool follow
 // simulators no room beside one another.
 bool go_tile_steps_fit(const go_domain* d) {
     const dim3 g = tile_grid(d->k);
-    return (int)(g.x * g.y) <= d->tile_steps_blocks;
+    const int most = (d->debug & GO_DEBUG_STEPS_ANY_SIZE) && d->tile_steps_blocks ? INT_MAX : d->tile_steps_blocks;
+    return (int)(g.x * g.y) <= most;
 }
 
-int go_launch_tile_steps(go_domain* d, cudaStream_t s, const StageArgs& a, int n) {
+// Where the process has too few SMs for the launch (a share of the device, say)
+// it is refused; the domain's steps then take one launch per stage: *done 0.
+int go_launch_tile_steps(go_domain* d, cudaStream_t s, const StageArgs& a, int n, bool* done) {
+    *done = true;
     if (n < 1) return GO_OK;
     StageArgs args = a;
     TileConst tc = tile_const(a.k);
     void* params[] = {&args, &tc, &n};
     d->stage_launches = 1;
-    cudaError_t e = allow_smem(d->device);
-    if (e == cudaSuccess)
-        e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(cdklm_tile_steps_kernel), tile_grid(a.k),
-                                        dim3(kTileThreads), params, sizeof(TileSmem), s);
+    const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(cdklm_tile_steps_kernel),
+                                                      tile_grid(a.k), dim3(kTileThreads), params, sizeof(TileSmem), s);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        d->tile_steps_blocks = 0;
+        *done = false;
+        return GO_OK;
+    }
     if (e != cudaSuccess) return go_fail(GO_ERR_CUDA, "step launch (tiles) failed: %s", cudaGetErrorString(e));
     return GO_OK;
 }
@@ -126,14 +131,13 @@ cudaError_t tile_batch_consts(const std::vector<StageArgs>& args, TileConst** ou
     std::vector<TileConst> h(args.size() / 2);
     for (size_t m = 0; m < h.size(); ++m) h[m] = tile_const(args[2 * m].k);
     *out = nullptr;
-    cudaError_t e = cudaMalloc(out, sizeof(TileConst) * h.size());
+    cudaError_t e = allow_smem(cdklm_tile_batch_kernel);
+    if (e == cudaSuccess) e = cudaMalloc(out, sizeof(TileConst) * h.size());
     if (e == cudaSuccess) e = cudaMemcpy(*out, h.data(), sizeof(TileConst) * h.size(), cudaMemcpyHostToDevice);
     return e;
 }
 
 cudaError_t tile_batch_launch(const TileBatchReq& r) {
-    const cudaError_t e = allow_smem(r.device);
-    if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr;
     const cudaLaunchConfig_t cfg = tile_config(dim3(r.ntiles), r.s, &attr, r.follows);
     return cudaLaunchKernelEx(&cfg, cdklm_tile_batch_kernel, r.args, r.dts, r.consts, r.tiles, r.rk_step);

@@ -630,8 +630,12 @@ int go_domain_stage_launches(go_domain* d, int* launches);
  * loads, so its bounded waits on the tiles' mbarriers run out; the stage
  * then sets GO_STATUS_TIMEOUT, leaves the region's cells unwritten and
  * returns, and the context stays usable.  Applies to stages prepared
- * after the call (a batch takes it from its members at go_batch_set_member). */
+ * after the call (a batch takes it from its members at go_batch_set_member).
+ * GO_DEBUG_STEPS_ANY_SIZE: a grid that runs the tile kernel asks for one
+ * cooperative launch of all steps whatever its size; one that does not fit
+ * on the device is refused at launch and takes one launch per stage. */
 #define GO_DEBUG_SKIP_TMA 0x1u
+#define GO_DEBUG_STEPS_ANY_SIZE 0x2u
 int go_domain_set_debug(go_domain* d, unsigned flags);
 
 /* Status words of every member of a batch (n values to status_host, member
