@@ -26,6 +26,8 @@ GO_STATUS_NONFINITE = 0x1
 GO_STATUS_ADJ_SCOPE = 0x2
 GO_STATUS_TIMEOUT = 0x4
 GO_STATUS_BOUNDS = 0x8
+GO_SHAPE_AUTO = -1
+GO_KERNEL_TILE = 9
 GO_DEBUG_SKIP_TMA = 0x1
 GO_DEBUG_STEPS_ANY_SIZE = 0x2
 GO_ERR_INVALID = -1
@@ -88,6 +90,7 @@ SIGNATURES = {
     "go_domain_set_wind_uniform": (_I, [_P, _F, _F, _F, _F]),
     "go_domain_set_wind_field": (_I, [_P, _P, _P, _P, _P, _I]),
     "go_domain_set_launch": (_I, [_P, _I, _I]),
+    "go_domain_kernel": (_I, [_P, ctypes.POINTER(_I), ctypes.POINTER(_I)]),
     "go_domain_set_arith": (_I, [_P, _I]),
     "go_check_quotients": (_I, [_P, _P, _P, _I, _P, _P]),
     "go_domain_set_land": (_I, [_P, _I]),
@@ -153,6 +156,7 @@ SIGNATURES = {
     "go_batch_destroy": (_I, [_P]),
     "go_batch_set_member": (_I, [_P, _I, _F, _P, _P, _P, _I, _P, _P, _P, _I, _P, _I, _F, _F]),
     "go_batch_set_launch": (_I, [_P, _I, _I, _I]),
+    "go_batch_kernel": (_I, [_P, ctypes.POINTER(_I), ctypes.POINTER(_I)]),
     "go_batch_set_arith": (_I, [_P, _I]),
     "go_batch_set_dt": (_I, [_P, _P, ctypes.POINTER(ctypes.c_float)]),
     "go_batch_tiles": (_I, [_P, ctypes.POINTER(_I)]),
@@ -245,6 +249,7 @@ class Domain:
         self.nx, self.ny = int(nx), int(ny)
         self.bc = tuple(int(b) for b in bc)
         self.bc_packed = pack_bc(*self.bc)
+        self.may_have_land = True
 
     def close(self):
         if getattr(self, "handle", None) is not None and self.handle.value:
@@ -284,11 +289,18 @@ class Domain:
     def set_launch(self, shape=0, rows_per_block=0):
         check(load().go_domain_set_launch(self.handle, int(shape), int(rows_per_block)))
 
+    def kernel(self):
+        """(launch shape or GO_KERNEL_TILE, rows per strip) the steps run now."""
+        k, r = ctypes.c_int(), ctypes.c_int()
+        check(load().go_domain_kernel(self.handle, ctypes.byref(k), ctypes.byref(r)))
+        return k.value, r.value
+
     def set_arith(self, mode):
         check(load().go_domain_set_arith(self.handle, int(mode)))
 
     def set_land(self, may_have_land):
         check(load().go_domain_set_land(self.handle, int(bool(may_have_land))))
+        self.may_have_land = bool(may_have_land)
 
     def status(self, clear=False):
         v = ctypes.c_uint32()
@@ -341,6 +353,13 @@ class Batch:
     def set_launch(self, shape=0, rows_per_block=0, blocks=0):
         check(load().go_batch_set_launch(self.handle, int(shape), int(rows_per_block), int(blocks)))
         self.launch = (int(shape), int(rows_per_block), int(blocks))
+
+    def kernel(self):
+        """(launch shape or GO_KERNEL_TILE, rows per strip) the steps run now;
+        every member has to be set."""
+        k, r = ctypes.c_int(), ctypes.c_int()
+        check(load().go_batch_kernel(self.handle, ctypes.byref(k), ctypes.byref(r)))
+        return k.value, r.value
 
     def set_arith(self, mode):
         check(load().go_batch_set_arith(self.handle, int(mode)))

@@ -112,6 +112,13 @@ static int auto_shape_land(int nx, int ny) {
     return (long long)nx * ny < 3500LL * 3500LL ? march_shape(nx, ny) : go_auto_shape(nx, ny);
 }
 
+// Default shape and strip height of a domain whose launch is left to the library.
+static void pick_launch(go_domain* d) {
+    if (!d->auto_launch) return;
+    d->shape = d->land_told ? auto_shape_land(d->k.nx, d->k.ny) : go_auto_shape(d->k.nx, d->k.ny);
+    d->rows_per_block = go_auto_rows(d->k.nx, d->k.ny, d->shape);
+}
+
 int go_friction_mode(const go_domain* d) {
     if (d->desc.friction_law == GO_FRICTION_LINEAR) return kFricLinear;
     return (d->k.r > 0.0f) ? kFricQuad : kFricNone;
@@ -256,11 +263,10 @@ int go_domain_create(const go_domain_desc* desc, go_domain** out) {
     k.V = s.dx / k.two_g;
     k.U = s.dy / k.two_g;
     k.two_r = two * s.r;
-    d->shape = go_auto_shape(s.nx, s.ny);
-    d->rows_per_block = go_auto_rows(s.nx, s.ny, d->shape);
     d->arith = GO_ARITH_RCP;
     d->has_land = 1;
     d->auto_launch = 1;
+    pick_launch(d);
     cudaError_t e = cudaGetDevice(&d->device);
     if (e == cudaSuccess) e = cudaMalloc(&d->d_frows, sizeof(float) * (s.ny + 4));
     if (e == cudaSuccess) e = cudaMemset(d->d_frows, 0, sizeof(float) * (s.ny + 4));
@@ -335,12 +341,25 @@ int go_domain_set_wind_field(go_domain* d, const float* x_cur, const float* x_ne
 
 int go_domain_set_launch(go_domain* d, int shape, int rows_per_block) {
     if (!d) return go_fail(GO_ERR_INVALID, "null domain");
+    if (shape == GO_SHAPE_AUTO && rows_per_block == 0) {
+        d->auto_launch = 1;
+        pick_launch(d);
+        return GO_OK;
+    }
     if (shape < 0 || shape > GO_SHAPE_PAIR) return go_fail(GO_ERR_INVALID, "launch shape %d (0..8)", shape);
     if (rows_per_block == 0) rows_per_block = go_auto_rows(d->k.nx, d->k.ny, shape);
     if (rows_per_block < 1) return go_fail(GO_ERR_INVALID, "rows_per_block must be >= 1");
     d->shape = shape;
     d->rows_per_block = rows_per_block;
     d->auto_launch = 0;
+    return GO_OK;
+}
+
+int go_domain_kernel(const go_domain* d, int* kernel, int* rows) {
+    if (!d || !kernel || !rows) return go_fail(GO_ERR_INVALID, "null argument");
+    const bool tile = go_tile_domain(d);
+    *kernel = tile ? GO_KERNEL_TILE : d->shape;
+    *rows = tile ? 0 : d->rows_per_block;
     return GO_OK;
 }
 
@@ -355,10 +374,7 @@ int go_domain_set_land(go_domain* d, int may_have_land) {
     if (!d) return go_fail(GO_ERR_INVALID, "null domain");
     d->has_land = may_have_land ? 1 : 0;
     d->land_told = d->has_land;
-    if (d->auto_launch) {
-        d->shape = d->land_told ? auto_shape_land(d->k.nx, d->k.ny) : go_auto_shape(d->k.nx, d->k.ny);
-        d->rows_per_block = go_auto_rows(d->k.nx, d->k.ny, d->shape);
-    }
+    pick_launch(d);
     return GO_OK;
 }
 

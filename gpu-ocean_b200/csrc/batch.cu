@@ -184,6 +184,65 @@ int batch_commit_pair(go_batch* b) {
     return GO_OK;
 }
 
+// Default shape and strip height of a batch whose launch is left to the library
+// (members that the tile kernel suits apart: batch_tile).
+void batch_pick(go_batch* b) {
+    const int n = b->n;
+    // 32-row strips (a batch launches enough blocks for long strips) and,
+    // once the tiles need more than one wave of blocks, the read-ahead shape
+    // with the less column work (measured on a B200, 100 members of 512^2:
+    // 1597 us per step with 128 x 5 blocks of 16 rows and register prefetch,
+    // 1532 with the ring, 1431 with 96-wide ring blocks and 32 rows).
+    b->rows = 32;
+    {
+        long long work5 = 0, work6 = 0;
+        for (int m = 0; m < n; ++m) {
+            const Scheme& k = b->members[m]->k;
+            work5 += shape_columns(5, k.nx) * k.ny;
+            work6 += shape_columns(6, k.nx) * k.ny;
+        }
+        const int ring = ring_shape(work5, work6);
+        long long tiles = 0;
+        for (int m = 0; m < n; ++m) {
+            const Scheme& k = b->members[m]->k;
+            tiles += shape_columns(ring, k.nx) / shape_block_width(ring) * ((k.ny + b->rows - 1) / b->rows);
+        }
+        b->shape = tiles > 148LL * shape_blocks_per_sm(ring) ? ring : 4;
+        // the column-pair kernel once the batch holds a few million cells
+        // (measured on a B200, us per step with the ring shape / the pair
+        // shape: 100 members of 512^2 1524 / 1145; 16 members 307 / 272;
+        // 4 members 123 / 125)
+        long long cells = 0;
+        for (int m = 0; m < n; ++m) cells += (long long)b->members[m]->k.nx * b->members[m]->k.ny;
+        if (cells >= kPairAutoBatchCells) {
+            // strip height by the cost of all members' strips (us per step,
+            // 32 rows / the height taken: 100 members of 195^2 276 / 245, 12
+            // of 700^2 311 / 269, 32 of 300^2 189 / 162)
+            b->shape = GO_SHAPE_PAIR;
+            double best = -1.0;
+            for (int r = 6; r <= 120; ++r) {
+                long long blocks = 0;
+                for (int m = 0; m < n; ++m) {
+                    const Scheme& k = b->members[m]->k;
+                    blocks += shape_columns(GO_SHAPE_PAIR, k.nx) / shape_block_width(GO_SHAPE_PAIR) *
+                              ((std::max(k.ny - 4, 1) + r - 1) / r);
+                }
+                const double cost = pair_strip_cost(blocks, r);
+                if (best < 0.0 || cost < best) { best = cost; b->rows = r; }
+            }
+        }
+        // with land, 16-row strips of the register-prefetch shape (a seventh of
+        // the corners land in patches; us per step, the choice above / this:
+        // 40 members of 512^2 796 / 685, 32 of 300^2 298 / 229, 8 of 1024^2
+        // 586 / 490, 60 of 128^2 155 / 138)
+        for (int m = 0; m < n; ++m)
+            if (b->members[m]->land_told) {
+                b->shape = 4;
+                b->rows = 16;
+            }
+    }
+}
+
 // Whether the batch runs the tile kernel: reciprocal quotients on north-up
 // grids, no land told, and members so narrow that the other kernels' whole
 // column blocks and frames cost more than its lower rate per cell.  The tile
@@ -592,59 +651,7 @@ int go_batch_create(go_domain* const* members, int n, go_batch** out) {
     const go_domain* d0 = members[0];
     b->variant = go_variant(d0);
     b->arith = d0->arith;
-    // 32-row strips (a batch launches enough blocks for long strips) and,
-    // once the tiles need more than one wave of blocks, the read-ahead shape
-    // with the less column work (measured on a B200, 100 members of 512^2:
-    // 1597 us per step with 128 x 5 blocks of 16 rows and register prefetch,
-    // 1532 with the ring, 1431 with 96-wide ring blocks and 32 rows).
-    b->rows = 32;
-    {
-        long long work5 = 0, work6 = 0;
-        for (int m = 0; m < n; ++m) {
-            const Scheme& k = members[m]->k;
-            work5 += shape_columns(5, k.nx) * k.ny;
-            work6 += shape_columns(6, k.nx) * k.ny;
-        }
-        const int ring = ring_shape(work5, work6);
-        long long tiles = 0;
-        for (int m = 0; m < n; ++m) {
-            const Scheme& k = members[m]->k;
-            tiles += shape_columns(ring, k.nx) / shape_block_width(ring) * ((k.ny + b->rows - 1) / b->rows);
-        }
-        b->shape = tiles > 148LL * shape_blocks_per_sm(ring) ? ring : 4;
-        // the column-pair kernel once the batch holds a few million cells
-        // (measured on a B200, us per step with the ring shape / the pair
-        // shape: 100 members of 512^2 1524 / 1145; 16 members 307 / 272;
-        // 4 members 123 / 125)
-        long long cells = 0;
-        for (int m = 0; m < n; ++m) cells += (long long)members[m]->k.nx * members[m]->k.ny;
-        if (cells >= kPairAutoBatchCells) {
-            // strip height by the cost of all members' strips (us per step,
-            // 32 rows / the height taken: 100 members of 195^2 276 / 245, 12
-            // of 700^2 311 / 269, 32 of 300^2 189 / 162)
-            b->shape = GO_SHAPE_PAIR;
-            double best = -1.0;
-            for (int r = 6; r <= 120; ++r) {
-                long long blocks = 0;
-                for (int m = 0; m < n; ++m) {
-                    const Scheme& k = members[m]->k;
-                    blocks += shape_columns(GO_SHAPE_PAIR, k.nx) / shape_block_width(GO_SHAPE_PAIR) *
-                              ((std::max(k.ny - 4, 1) + r - 1) / r);
-                }
-                const double cost = pair_strip_cost(blocks, r);
-                if (best < 0.0 || cost < best) { best = cost; b->rows = r; }
-            }
-        }
-        // with land, 16-row strips of the register-prefetch shape (a seventh of
-        // the corners land in patches; us per step, the choice above / this:
-        // 40 members of 512^2 796 / 685, 32 of 300^2 298 / 229, 8 of 1024^2
-        // 586 / 490, 60 of 128^2 155 / 138)
-        for (int m = 0; m < n; ++m)
-            if (members[m]->land_told) {
-                b->shape = 4;
-                b->rows = 16;
-            }
-    }
+    batch_pick(b);
     for (int m = 0; m < n; ++m) {
         const go_domain* d = members[m];
         if (go_has_open_bc(d)) {
@@ -718,6 +725,14 @@ int go_batch_set_member(go_batch* b, int m, float dt, float* eta0, float* hu0, f
 
 int go_batch_set_launch(go_batch* b, int shape, int rows_per_block, int blocks) {
     if (!b) return go_fail(GO_ERR_INVALID, "null batch");
+    if (shape == GO_SHAPE_AUTO && rows_per_block == 0 && blocks == 0) {
+        b->auto_launch = true;
+        b->blocks = 0;
+        batch_pick(b);
+        b->dirty = true;
+        drop_graph(b);
+        return GO_OK;
+    }
     if (shape < 0 || shape > GO_SHAPE_PAIR) return go_fail(GO_ERR_INVALID, "launch shape %d (0..8)", shape);
     if (rows_per_block == 0) rows_per_block = 32;
     if (rows_per_block < 1 || blocks < 0) return go_fail(GO_ERR_INVALID, "rows_per_block >= 1, blocks >= 0");
@@ -727,6 +742,15 @@ int go_batch_set_launch(go_batch* b, int shape, int rows_per_block, int blocks) 
     b->auto_launch = false;
     b->dirty = true;
     drop_graph(b);
+    return GO_OK;
+}
+
+int go_batch_kernel(go_batch* b, int* kernel, int* rows) {
+    if (!b || !kernel || !rows) return go_fail(GO_ERR_INVALID, "null argument");
+    const int rc = batch_commit(b);
+    if (rc) return rc;
+    *kernel = b->tile ? GO_KERNEL_TILE : b->shape;
+    *rows = b->tile ? 0 : b->rows;
     return GO_OK;
 }
 

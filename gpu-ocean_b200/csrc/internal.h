@@ -82,8 +82,9 @@ go::Variant go_variant(const go_domain* d);
 int go_launch_stage(go_domain* d, cudaStream_t s, const go::StageArgs& a, bool follows = false);
 
 // Tile stage kernel (tile_launch.cu): set-up of a domain that may run it,
-// whether a stage does, and its launches.
+// whether its stages do (the arrays' offsets apart), whether a stage does, and its launches.
 int go_tile_setup(go_domain* d);
+bool go_tile_domain(const go_domain* d);
 bool go_tile_stage(const go_domain* d, const go::StageArgs& a);
 int go_launch_tile(go_domain* d, cudaStream_t s, const go::StageArgs& a, bool follows);
 bool go_tile_steps_fit(const go_domain* d);

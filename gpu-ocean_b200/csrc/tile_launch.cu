@@ -64,11 +64,13 @@ int go_tile_setup(go_domain* d) {
 // 70.8 / 99.6 but 71.0 / 68.1.  With land (a seventh of the corners, in patches
 // of 20 cells, so that few tiles are deep): 512^2 23.7 / 33.0 and 18.4 / 23.6,
 // 640^2 34.4 / 39.3 but 26.5 / 24.6, 1024^2 68.9 / 78.1 but 63.9 / 52.5.
-bool go_tile_stage(const go_domain* d, const StageArgs& a) {
-    const long long cells = (long long)a.k.nx * a.k.ny;
+bool go_tile_domain(const go_domain* d) {
+    const long long cells = (long long)d->k.nx * d->k.ny;
     return d->auto_launch && cells < (d->land_told ? kTileLandCells : kTileCells) && d->arith == GO_ARITH_RCP &&
-           !go_general_north(d) && offsets_fit(a);
+           !go_general_north(d);
 }
+
+bool go_tile_stage(const go_domain* d, const StageArgs& a) { return go_tile_domain(d) && offsets_fit(a); }
 
 // One stage.  follows: the launch before it on the stream is a tile stage of
 // the same call, so this one is a programmatic dependent launch: its blocks

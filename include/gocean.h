@@ -303,9 +303,15 @@ int go_sample_wind(void* stream, const float* field, int w, int h, int nx, int n
  * kernel (32 x 16 cells per block) below 1.15 million cells, or 350 thousand
  * where go_domain_set_land told of land; else shape 8 from 1.15 million cells,
  * or 3500^2 with land; else shape 5, 6 or 4 by the columns they compute.
- * Chosen by the autotuner among the shapes; every kernel computes identical
+ * GO_SHAPE_AUTO (with 0 rows) returns a domain to that choice.
+ * Chosen by the autotuner among these; every kernel computes identical
  * results. */
+#define GO_SHAPE_AUTO (-1)
 int go_domain_set_launch(go_domain* d, int shape, int rows_per_block);
+/* The kernel that go_cdklm_step runs as the domain is set now: a launch shape
+ * or GO_KERNEL_TILE, and its rows per strip (0 with the tile kernel). */
+#define GO_KERNEL_TILE 9
+int go_domain_kernel(const go_domain* d, int* kernel, int* rows);
 /* Shape 8: the column-pair kernel.  Blocks of 64 threads, each thread two
  * adjacent columns in packed FP32x2 arithmetic (sm_100 FADD2/FFMA2), inputs
  * of the boundary-free blocks staged through shared memory by TMA tile
@@ -407,8 +413,11 @@ int go_batch_set_member(go_batch* b, int m, float dt, float* eta0, float* hu0, f
  * tile list.  A batch that this call was never made for takes the tile kernel
  * for narrow members and otherwise shape 8 with the strip height that suits
  * all members' strips, or 4 with few cells in all, one block per tile; shape 4
- * with 16-row strips where a member was told that it may have land. */
+ * with 16-row strips where a member was told that it may have land.
+ * GO_SHAPE_AUTO (with 0 rows and blocks) returns a batch to that choice. */
 int go_batch_set_launch(go_batch* b, int shape, int rows_per_block, int blocks);
+/* The kernel of a batch whose members are all set (as go_domain_kernel). */
+int go_batch_kernel(go_batch* b, int* kernel, int* rows);
 int go_batch_set_arith(go_batch* b, int mode);
 
 /* New per-member time steps (n floats, host).  A captured graph reads them
