@@ -92,31 +92,69 @@ static int march_shape(int nx, int ny) {
     return blocks > 148LL * go::shape_blocks_per_sm(ring) ? ring : 4;
 }
 
-// Default launch shape of the grids that the tile kernel leaves (go_tile_stage):
-// the column-pair kernel (shape 8) from about 1070^2 cells up.  Measured on a
-// B200, us per step, best of shapes 4 .. 6 / shape 8 (walls N/S, periodic E/W),
-// one simulator and three on their own streams: 1280^2 100 / 87 and 68 / 60,
-// 1501 x 1203 109 / 99 and 75 / 68, 2048^2 203 / 174 and 164 / 135, 4096^2
-// 684 / 584 and 641 / 528.
-int go_auto_shape(int nx, int ny) {
-    if ((long long)nx * ny >= kPairAutoCells) return GO_SHAPE_PAIR;
-    return march_shape(nx, ny);
+// Cells from which a domain's stages run the column-pair kernel.  Its blocks at
+// closed (wall) east and west sides are part of the boundary frame, which costs
+// several times a block of the region, more so with a per-cell wind; land
+// costs its two-column warps more than the marching kernel's.  Measured on a B200,
+// us per step, marching (best of shapes 5 and 6) / column pairs; one simulator and
+// three on their own streams; island: 1% of the corners, patches: a seventh:
+//   periodic east-west, uniform wind: 1152^2 80 / 81 and 57 / 50, 1536^2 127 / 114
+//     and 98 / 80, 2048^2 203 / 171 and 164 / 134, 4096^2 684 / 581 and 641 / 521;
+//     with patches 1152^2 92 / 99 and 67 / 68, 1536^2 152 / 144 and 118 / 109,
+//     2048^2 239 / 221 and 198 / 181, 4096^2 821 / 785 and 778 / 705;
+//   the same, per-cell wind: 1152^2 88 / 90 and 75 / 75, 1536^2 169 / 147 and 132 / 123;
+//     with patches 1152^2 100 / 110 and 87 / 91, 1536^2 192 / 178 and 154 / 151;
+//   closed, uniform wind: 1152^2 79 / 91 and 57 / 63, 1536^2 125 / 119 and 97 / 101,
+//     2048^2 198 / 189 and 163 / 162; with an island 2048^2 210 / 212 and 175 / 186,
+//     3072^2 423 / 389 and 380 / 378; with patches 2048^2 236 / 258 and 197 / 235,
+//     3072^2 483 / 491 and 431 / 479;
+//   closed, per-cell wind: 1152^2 84 / 115 and 74 / 96, 1536^2 166 / 187 and 130 / 148;
+//     with an island 2048^2 265 / 302 and 233 / 256, 3072^2 582 / 565 and 505 / 541;
+//     with patches 3072^2 645 / 665 and 562 / 634, 4096^2 1064 / 1128 and 1024 / 1085.
+// Where land was neither told of nor ruled out, for rotated grids, IEEE
+// quotients and open boundaries, which those figures do not cover: from 1500^2.
+static long long pair_cells(const go_domain* d) {
+    const long long usual = 1500LL * 1500LL;
+    if (d->arith != GO_ARITH_RCP || go_general_north(d) || go_has_open_bc(d)) return usual;
+    const bool closed = d->k.bcE == kWall || d->k.bcW == kWall, field = d->wx_cur != nullptr;
+    if (closed && d->land_told) return field ? 3500LL * 3500LL : 2300LL * 2300LL;
+    if (!closed && d->land_ruled_out) return field ? 1500LL * 1000LL : 1150LL * 1000LL;
+    return usual;
 }
 
-// The same for bathymetry with land, whose branches cost the two-column warps of
-// the column-pair kernel more: the marching kernel up to 3500^2 cells (per-cell
-// wind, a seventh of the corners land in patches of 20 cells; best of shapes
-// 4 .. 6 / shape 8: 1536^2 149 / 166 and 112 / 160, 2048^2 228 / 268 and 188 / 220,
-// 3072^2 467 / 487 and 411 / 446, 4096^2 786 / 779 and 740 / 754).
-static int auto_shape_land(int nx, int ny) {
-    return (long long)nx * ny < 3500LL * 3500LL ? march_shape(nx, ny) : go_auto_shape(nx, ny);
+// Default launch shape of the stages that the tile kernel leaves (go_tile_stage).
+int go_auto_shape(const go_domain* d) {
+    const int nx = d->k.nx, ny = d->k.ny;
+    return (long long)nx * ny >= pair_cells(d) ? GO_SHAPE_PAIR : march_shape(nx, ny);
+}
+
+// Grids that run the tile kernel unless a launch shape was set.  Measured on a
+// B200, us per RK2 step, tile against the marching kernel's default; one
+// simulator, and three on their own streams: 512^2 17.2 / 28.8 and 11.7 / 18.9,
+// 768^2 30.7 / 46.3 and 23.8 / 29.5, 1024^2 48.8 / 67.1 and 44.6 / 46.4, 1280^2
+// 70.8 / 99.6 but 71.0 / 68.1.  With land (a seventh of the corners, in patches
+// of 20 cells, so that few tiles are deep): 512^2 23.7 / 33.0 and 18.4 / 23.6,
+// 640^2 34.4 / 39.3 but 26.5 / 24.6, 1024^2 68.9 / 78.1 but 63.9 / 52.5.  Land
+// that was neither told of nor ruled out counts as land.
+bool go_tile_domain(const go_domain* d) {
+    const long long cells = (long long)d->k.nx * d->k.ny;
+    return d->auto_launch && cells < (d->land_ruled_out ? kTileCells : 350LL * 1000LL) && d->arith == GO_ARITH_RCP &&
+           !go_general_north(d);
 }
 
 // Default shape and strip height of a domain whose launch is left to the library.
 static void pick_launch(go_domain* d) {
     if (!d->auto_launch) return;
-    d->shape = d->land_told ? auto_shape_land(d->k.nx, d->k.ny) : go_auto_shape(d->k.nx, d->k.ny);
+    d->shape = go_auto_shape(d);
     d->rows_per_block = go_auto_rows(d->k.nx, d->k.ny, d->shape);
+}
+
+// Per-cell wind arrays, or null ones for uniform wind, whose kind the default
+// launch depends on.
+static void set_wind_arrays(go_domain* d, const float* xc, const float* xn, const float* yc, const float* yn) {
+    const bool other = (xc != nullptr) != (d->wx_cur != nullptr);
+    d->wx_cur = xc; d->wx_next = xn; d->wy_cur = yc; d->wy_next = yn;
+    if (other) pick_launch(d);
 }
 
 int go_friction_mode(const go_domain* d) {
@@ -320,7 +358,7 @@ int go_domain_set_coriolis(go_domain* d, const float* f_rows_host, int n) {
 int go_domain_set_wind_uniform(go_domain* d, float x_cur, float x_next, float y_cur, float y_next) {
     if (!d) return go_fail(GO_ERR_INVALID, "null domain");
     d->wxc = x_cur; d->wxn = x_next; d->wyc = y_cur; d->wyn = y_next;
-    d->wx_cur = d->wx_next = d->wy_cur = d->wy_next = nullptr;
+    set_wind_arrays(d, nullptr, nullptr, nullptr, nullptr);
     return GO_OK;
 }
 
@@ -328,13 +366,13 @@ int go_domain_set_wind_field(go_domain* d, const float* x_cur, const float* x_ne
                              const float* y_cur, const float* y_next, int pitch) {
     if (!d) return go_fail(GO_ERR_INVALID, "null domain");
     if (!x_cur && !x_next && !y_cur && !y_next) {
-        d->wx_cur = d->wx_next = d->wy_cur = d->wy_next = nullptr;
+        set_wind_arrays(d, nullptr, nullptr, nullptr, nullptr);
         return GO_OK;
     }
     if (!x_cur || !x_next || !y_cur || !y_next) return go_fail(GO_ERR_INVALID, "wind field needs four arrays");
     int rc = go_check_pitch(pitch, d->k.nx, "wind");
     if (rc) return rc;
-    d->wx_cur = x_cur; d->wx_next = x_next; d->wy_cur = y_cur; d->wy_next = y_next;
+    set_wind_arrays(d, x_cur, x_next, y_cur, y_next);
     d->wpitch = pitch / 4;
     return GO_OK;
 }
@@ -367,6 +405,7 @@ int go_domain_set_arith(go_domain* d, int mode) {
     if (!d) return go_fail(GO_ERR_INVALID, "null domain");
     if (mode != GO_ARITH_EXACT && mode != GO_ARITH_RCP) return go_fail(GO_ERR_INVALID, "arith mode %d", mode);
     d->arith = mode;
+    pick_launch(d);
     return GO_OK;
 }
 
@@ -374,6 +413,7 @@ int go_domain_set_land(go_domain* d, int may_have_land) {
     if (!d) return go_fail(GO_ERR_INVALID, "null domain");
     d->has_land = may_have_land ? 1 : 0;
     d->land_told = d->has_land;
+    d->land_ruled_out = !d->has_land;
     pick_launch(d);
     return GO_OK;
 }

@@ -38,6 +38,7 @@ struct go_domain {
     int auto_launch;         // launch choice left to the library (until a shape is set)
     int land_told;           // go_domain_set_land said that the bathymetry may hold land
     int tile_steps_blocks;   // most tiles of a cooperative launch of many steps (0: none)
+    int land_ruled_out;      // go_domain_set_land said that the bathymetry holds no land
 };
 
 // Records the message of a failed call (go_last_error) and returns code.
@@ -56,7 +57,7 @@ int go_check_pitch(int pitch_bytes, int min_floats, const char* what);
 // in [2, 16] nearest below (column strips x ny) / 600, so that small grids
 // still launch enough blocks to cover the 148 SMs.
 int go_auto_rows(int nx, int ny, int shape);
-int go_auto_shape(int nx, int ny);
+int go_auto_shape(const go_domain* d);
 // Open kinds (codes 3/4) of one axis (csrc/open_boundaries.cu).
 int go_open_bc_ns(const go_domain* d, cudaStream_t s, float* h, float* u, float* v, int p);
 int go_open_bc_ew(const go_domain* d, cudaStream_t s, float* h, float* u, float* v, int p);
@@ -83,6 +84,7 @@ int go_launch_stage(go_domain* d, cudaStream_t s, const go::StageArgs& a, bool f
 
 // Tile stage kernel (tile_launch.cu): set-up of a domain that may run it,
 // whether its stages do (the arrays' offsets apart), whether a stage does, and its launches.
+constexpr long long kTileCells = 1150LL * 1000LL;   // grids of this many cells and more never run it
 int go_tile_setup(go_domain* d);
 bool go_tile_domain(const go_domain* d);
 bool go_tile_stage(const go_domain* d, const go::StageArgs& a);

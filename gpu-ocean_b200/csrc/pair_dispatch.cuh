@@ -23,9 +23,8 @@ constexpr int kPairMinBlocksFrame = 6;
 constexpr int kPairSlots = 2;
 constexpr int kPairUnroll = 1;
 constexpr int kPairFrameRows = 8;
-// default-shape thresholds: a grid of at least this many cells, a batch
-// whose members hold at least this many together
-constexpr long long kPairAutoCells = 1150LL * 1000LL;
+// a batch whose members hold at least this many cells together runs the
+// column-pair kernel by default
 constexpr long long kPairAutoBatchCells = 2LL << 20;
 
 // The block grid of an nx x ny domain (see PairGrid): the region of TMA

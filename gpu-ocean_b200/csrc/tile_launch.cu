@@ -11,8 +11,6 @@ using namespace go;
 
 namespace {
 
-constexpr long long kTileCells = 1150LL * 1000LL, kTileLandCells = 350LL * 1000LL;
-
 dim3 tile_grid(const Scheme& k) { return dim3((k.nx + kTileX - 1) / kTileX, (k.ny + kTileY - 1) / kTileY); }
 
 // Allows a kernel its shared-memory size in the current context.  Done for
@@ -55,19 +53,6 @@ int go_tile_setup(go_domain* d) {
                                                           sizeof(TileSmem)));
     d->tile_steps_blocks = coop && per_sm > 0 ? sms : 0;
     return GO_OK;
-}
-
-// Grids that run the tile kernel unless a launch shape was set.  Measured on a
-// B200, us per RK2 step, tile against the marching kernel's default; one
-// simulator, and three on their own streams: 512^2 17.2 / 28.8 and 11.7 / 18.9,
-// 768^2 30.7 / 46.3 and 23.8 / 29.5, 1024^2 48.8 / 67.1 and 44.6 / 46.4, 1280^2
-// 70.8 / 99.6 but 71.0 / 68.1.  With land (a seventh of the corners, in patches
-// of 20 cells, so that few tiles are deep): 512^2 23.7 / 33.0 and 18.4 / 23.6,
-// 640^2 34.4 / 39.3 but 26.5 / 24.6, 1024^2 68.9 / 78.1 but 63.9 / 52.5.
-bool go_tile_domain(const go_domain* d) {
-    const long long cells = (long long)d->k.nx * d->k.ny;
-    return d->auto_launch && cells < (d->land_told ? kTileLandCells : kTileCells) && d->arith == GO_ARITH_RCP &&
-           !go_general_north(d);
 }
 
 bool go_tile_stage(const go_domain* d, const StageArgs& a) { return go_tile_domain(d) && offsets_fit(a); }

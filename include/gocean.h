@@ -299,10 +299,13 @@ int go_sample_wind(void* stream, const float* field, int w, int h, int nx, int n
  * in {2, 4, 8, 16, 24} that minimises whole waves of blocks times the strip
  * length plus its 4 recomputed halo rows; for shape 8 a multiple of 3 by a fit
  * to measured heights).  A domain that this call was never made for takes its
- * kernel from its size: with reciprocal quotients on a north-up grid the tile
- * kernel (32 x 16 cells per block) below 1.15 million cells, or 350 thousand
- * where go_domain_set_land told of land; else shape 8 from 1.15 million cells,
- * or 3500^2 with land; else shape 5, 6 or 4 by the columns they compute.
+ * kernel from its size, its east and west sides, its wind kind and what
+ * go_domain_set_land told: with reciprocal quotients on a north-up grid the
+ * tile kernel (32 x 16 cells per block) below 350 thousand cells, or 1.15
+ * million where land was ruled out; then, with one thread per column, shape 5, 6
+ * or 4 by the columns they compute; and shape 8 from 1500^2 cells, from 1.15
+ * million (1.5 million with per-cell wind) with periodic east and west sides and
+ * land ruled out, and from 2300^2 (3500^2) with land and a closed side.
  * GO_SHAPE_AUTO (with 0 rows) returns a domain to that choice.
  * Chosen by the autotuner among these; every kernel computes identical
  * results. */

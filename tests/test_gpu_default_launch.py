@@ -59,3 +59,45 @@ def test_batch_returns_to_the_default(n, nx, kernel):
     torch.cuda.synchronize()
     for a, b in zip(sims[n // 2].download(), ref.download()):
         assert np.array_equal(a, b)
+
+
+CLOSED, PERIODIC = (1, 1, 1, 1), (1, 2, 1, 2)
+
+
+def _domain_kernel(nx, ny, bc, land, field, exact=False, north=(0.0, 1.0)):
+    dom = _native.Domain(nx, ny, 1000.0, 1000.0, 9.81, bc=bc, north=north)
+    if land is not None:
+        dom.set_land(land)
+    if exact:
+        dom.set_arith(_native.GO_ARITH_EXACT)
+    if field:
+        w = torch.zeros((ny, nx), device="cuda")
+        dom.set_wind_field(w, w, w, w)
+        before = dom.kernel()
+        dom.set_wind_uniform(0.0, 0.0, 0.0, 0.0)
+        dom.set_wind_field(w, w, w, w)               # the choice follows the wind kind
+        assert dom.kernel() == before
+    return dom.kernel()[0]
+
+
+@pytest.mark.parametrize("nx,ny,bc,land,field,kernel", [
+    (500, 500, CLOSED, None, False, TILE), (500, 500, CLOSED, True, True, TILE), (700, 700, CLOSED, None, False, "march"),
+    (700, 700, PERIODIC, True, False, "march"), (700, 700, CLOSED, False, True, TILE),
+    (1300, 1100, PERIODIC, None, False, "march"), (1300, 1100, PERIODIC, False, False, PAIR),
+    (1300, 1100, PERIODIC, False, True, "march"), (1300, 1200, PERIODIC, False, True, PAIR),
+    (1300, 1100, CLOSED, False, False, "march"), (1300, 1100, PERIODIC, True, False, "march"),
+    (1600, 1600, PERIODIC, None, False, PAIR), (1600, 1600, CLOSED, None, True, PAIR),
+    (1600, 1600, PERIODIC, True, True, PAIR), (1600, 1600, CLOSED, False, True, PAIR),
+    (1600, 1600, CLOSED, True, False, "march"), (2400, 2400, CLOSED, True, False, PAIR),
+    (2400, 2400, CLOSED, True, True, "march"), (3600, 3600, CLOSED, True, True, PAIR)])
+def test_default_kernel_by_sides_land_and_wind(nx, ny, bc, land, field, kernel):
+    got = _domain_kernel(nx, ny, bc, land, field)
+    assert got == kernel or (kernel == "march" and got in (4, 5, 6))
+
+
+def test_default_kernel_of_the_forms_it_was_not_measured_for():
+    """IEEE quotients and rotated grids: as before land was asked about."""
+    for kw in (dict(exact=True), dict(north=(0.6, 0.8))):
+        assert _domain_kernel(500, 500, CLOSED, False, False, **kw) in (4, 5, 6)
+        assert _domain_kernel(1300, 1100, PERIODIC, False, False, **kw) in (4, 5, 6)
+        assert _domain_kernel(1600, 1600, CLOSED, True, True, **kw) == PAIR
