@@ -69,6 +69,7 @@ struct go_batch {
     // tile kernel: the default launch (until go_batch_set_launch) of members
     // it suits (batch_tile)
     bool auto_launch = true, tile = false;
+    int picked = -1;                   // wind and arithmetic kind that the default shape was chosen for
     TileConst* d_tile_consts = nullptr;
     int arith = 0;
     Variant variant;
@@ -188,6 +189,9 @@ int batch_commit_pair(go_batch* b) {
 // (members that the tile kernel suits apart: batch_tile).
 void batch_pick(go_batch* b) {
     const int n = b->n;
+    const bool field = b->args[0].wx_cur != nullptr, plain = b->arith == GO_ARITH_RCP && !b->variant.gen_north;
+    if (b->picked == field + 2 * plain) return;
+    b->picked = field + 2 * plain;
     // 32-row strips (a batch launches enough blocks for long strips) and,
     // once the tiles need more than one wave of blocks, the read-ahead shape
     // with the less column work (measured on a B200, 100 members of 512^2:
@@ -231,15 +235,30 @@ void batch_pick(go_batch* b) {
                 if (best < 0.0 || cost < best) { best = cost; b->rows = r; }
             }
         }
-        // with land, 16-row strips of the register-prefetch shape (a seventh of
-        // the corners land in patches; us per step, the choice above / this:
-        // 40 members of 512^2 796 / 685, 32 of 300^2 298 / 229, 8 of 1024^2
-        // 586 / 490, 60 of 128^2 155 / 138)
-        for (int m = 0; m < n; ++m)
-            if (b->members[m]->land_told) {
-                b->shape = 4;
-                b->rows = 16;
-            }
+        // With land, 16-row strips of the register-prefetch shape where the
+        // column-pair kernel does not pay: batches below its size, and those of
+        // closed (wall) east or west sides, whose column blocks are frame there,
+        // unless little of the water is beside land (us per step on a B200, 32-row
+        // pair strips / this; patches: a seventh of the land members' corners,
+        // island: 1%).  Closed sides, uniform wind: 100 members of 512^2, patches
+        // in all 1870 / 1694, in half 1686 / 1624, in two 1533 / 1560, 32 of 300^2
+        // all 319 / 235, 12 of 700^2 all 409 / 379, one 342 / 348; per-cell wind: 100
+        // of 512^2 two 2259 / 2051, 12 of 700^2 islands in all 484 / 464.  Periodic
+        // sides: 100 of 512^2 all 1449 / 1788, two 1212 / 1669, per-cell wind all
+        // 1887 / 2278, 8 of 1024^2 all 467 / 523.  Below: 4 of 512^2 all 141 (32-row
+        // strips) / 105, 8 of 256^2 131 / 83.  (Rotated grids and IEEE quotients,
+        // not measured, keep the shape without land.)
+        long long land = 0, closed = 0;
+        for (int m = 0; m < n; ++m) {
+            const go_domain* d = b->members[m];
+            const long long c = (long long)d->k.nx * d->k.ny;
+            if (d->land_told) land += c;
+            if (d->k.bcE == kWall || d->k.bcW == kWall) closed += c;
+        }
+        if (land > 0 && plain && (cells < kPairAutoBatchCells || (2 * closed >= cells && (field || 4 * land >= cells)))) {
+            b->shape = 4;
+            b->rows = 16;
+        }
     }
 }
 
@@ -294,6 +313,7 @@ int batch_lay_out(go_batch* b) {
         if (!b->member_set[m]) return go_fail(GO_ERR_INVALID, "batch member %d has no state set", m);
     int rc = batch_variant(b);
     if (rc) return rc;
+    if (b->auto_launch) batch_pick(b);
     Variant v = b->variant;
     v.shape = b->shape;
     v.rcp = b->arith == GO_ARITH_RCP;
@@ -651,7 +671,6 @@ int go_batch_create(go_domain* const* members, int n, go_batch** out) {
     const go_domain* d0 = members[0];
     b->variant = go_variant(d0);
     b->arith = d0->arith;
-    batch_pick(b);
     for (int m = 0; m < n; ++m) {
         const go_domain* d = members[m];
         if (go_has_open_bc(d)) {
@@ -728,7 +747,7 @@ int go_batch_set_launch(go_batch* b, int shape, int rows_per_block, int blocks) 
     if (shape == GO_SHAPE_AUTO && rows_per_block == 0 && blocks == 0) {
         b->auto_launch = true;
         b->blocks = 0;
-        batch_pick(b);
+        b->picked = -1;
         b->dirty = true;
         drop_graph(b);
         return GO_OK;

@@ -414,9 +414,11 @@ int go_batch_set_member(go_batch* b, int m, float dt, float* eta0, float* hu0, f
 /* Launch shape (as go_domain_set_launch) and persistent grid size: blocks
  * = 0 launches one block per tile, blocks > 0 that many blocks walking the
  * tile list.  A batch that this call was never made for takes the tile kernel
- * for narrow members and otherwise shape 8 with the strip height that suits
- * all members' strips, or 4 with few cells in all, one block per tile; shape 4
- * with 16-row strips where a member was told that it may have land.
+ * for narrow members and otherwise shape 8, with the strip height that suits
+ * all members' strips, or 4 to 6 with few cells in all, one block per tile.  With
+ * members that were told of land, shape 4 with 16-row strips runs batches of few
+ * cells, and those of closed east or west sides unless a uniform wind and few
+ * such members speak for shape 8.
  * GO_SHAPE_AUTO (with 0 rows and blocks) returns a batch to that choice. */
 int go_batch_set_launch(go_batch* b, int shape, int rows_per_block, int blocks);
 /* The kernel of a batch whose members are all set (as go_domain_kernel). */

@@ -101,3 +101,45 @@ def test_default_kernel_of_the_forms_it_was_not_measured_for():
         assert _domain_kernel(500, 500, CLOSED, False, False, **kw) in (4, 5, 6)
         assert _domain_kernel(1300, 1100, PERIODIC, False, False, **kw) in (4, 5, 6)
         assert _domain_kernel(1600, 1600, CLOSED, True, True, **kw) == PAIR
+
+
+def _members(n, nx, land, bc, field=False):
+    """n flat-bottomed members, the first `land` of them told of land."""
+    ctx, sims = Common.CUDAContext(), []
+    from SWESimulators import WindStress
+    shape = (3, 4) if field else (1, 1)
+    rng = np.random.default_rng(1)
+    for m in range(n):
+        H = np.full((nx + 5, nx + 5), 50.0, np.float32)
+        if m < land:
+            H[nx // 3:nx // 3 + 6, nx // 2:nx // 2 + 8] = 1.0e20
+        eta, hu, hv = (rng.standard_normal((nx + 4, nx + 4)).astype(np.float32) * s for s in (0.1, 1.0, 1.0))
+        wind = WindStress.WindStress(t=[0], X=[np.full(shape, 1e-4, np.float32)], Y=[np.full(shape, 1e-4, np.float32)])
+        sims.append(CDKLM16.CDKLM16(ctx, eta, hu, hv, H, nx, nx, 1000.0, 1000.0, 5.0, 9.81, 1.2e-4, 0.0,
+                                    boundary_conditions=Common.BoundaryConditions(*bc), wind_stress=wind))
+    return sims
+
+
+@pytest.mark.parametrize("land,bc,field,kernel", [
+    (0, PERIODIC, False, (PAIR, None)), (1, PERIODIC, False, (PAIR, None)), (12, PERIODIC, True, (PAIR, None)),
+    (1, CLOSED, False, (PAIR, None)), (3, CLOSED, False, (4, 16)), (12, CLOSED, False, (4, 16)),
+    (1, CLOSED, True, (4, 16)), (0, CLOSED, True, (PAIR, None))])
+def test_default_kernel_of_batches_with_land(land, bc, field, kernel):
+    sims = _members(12, 420, land, bc, field)
+    ens = BatchedEnsemble.BatchedCDKLM16(sims)
+    got = ens.batch.kernel()
+    assert got[0] == kernel[0] and kernel[1] in (None, got[1])
+    if (land, bc) in ((1, PERIODIC), (1, CLOSED)) and not field:
+        ens.advance(3)                       # a land member among others without: each as alone
+        alone = [s for s in _members(2, 420, 1, bc)]
+        for s in alone:
+            s._domain.set_launch(4, 8)
+            s.step(3.0 * float(np.float32(s.dt)))
+        torch.cuda.synchronize()
+        for s, w in zip(sims, alone):
+            for a, b in zip(s.download(), w.download()):
+                assert np.array_equal(a, b)
+
+
+def test_default_kernel_of_small_batches_with_land():
+    assert BatchedEnsemble.BatchedCDKLM16(_members(4, 420, 1, PERIODIC)).batch.kernel() == (4, 16)
