@@ -219,18 +219,24 @@ void batch_pick(go_batch* b) {
         long long cells = 0;
         for (int m = 0; m < n; ++m) cells += (long long)b->members[m]->k.nx * b->members[m]->k.ny;
         if (cells >= kPairAutoBatchCells) {
-            // strip height by the cost of all members' strips (us per step,
-            // 32 rows / the height taken: 100 members of 195^2 276 / 245, 12
-            // of 700^2 311 / 269, 32 of 300^2 189 / 162)
+            // strip height by the cost of all members' region strips (us per step,
+            // 32 rows / the height taken: periodic sides, 100 members of 195^2 276 /
+            // 245, 12 of 700^2 311 / 269, 32 of 300^2 189 / 162; closed ones, whose
+            // outer column blocks are frame, 12 of 700^2 312 / 303, 32 of 300^2 234 /
+            // 210, 16 of 512^2 278 / 267).  Without region strips (closed sides and
+            // at most two column blocks) the height says nothing.
             b->shape = GO_SHAPE_PAIR;
+            std::vector<long long> columns(n);
+            for (int m = 0; m < n; ++m) {
+                const PairGrid g = pair_grid(b->members[m]->k, b->rows, true);
+                columns[m] = g.bx1 - g.bx0;
+            }
             double best = -1.0;
             for (int r = 6; r <= 120; ++r) {
                 long long blocks = 0;
-                for (int m = 0; m < n; ++m) {
-                    const Scheme& k = b->members[m]->k;
-                    blocks += shape_columns(GO_SHAPE_PAIR, k.nx) / shape_block_width(GO_SHAPE_PAIR) *
-                              ((std::max(k.ny - 4, 1) + r - 1) / r);
-                }
+                for (int m = 0; m < n; ++m)
+                    blocks += columns[m] * ((std::max(b->members[m]->k.ny - 4, 1) + r - 1) / r);
+                if (blocks == 0) break;
                 const double cost = pair_strip_cost(blocks, r);
                 if (best < 0.0 || cost < best) { best = cost; b->rows = r; }
             }

@@ -143,3 +143,10 @@ def test_default_kernel_of_batches_with_land(land, bc, field, kernel):
 
 def test_default_kernel_of_small_batches_with_land():
     assert BatchedEnsemble.BatchedCDKLM16(_members(4, 420, 1, PERIODIC)).batch.kernel() == (4, 16)
+
+
+@pytest.mark.parametrize("n,nx,bc,rows", [(12, 700, CLOSED, 29), (12, 700, PERIODIC, 22), (40, 240, CLOSED, 32)])
+def test_strip_heights_of_batches_count_the_region_strips(n, nx, bc, rows):
+    """Closed east and west sides: the outer column blocks are frame, and with
+    two column blocks there are no others."""
+    assert BatchedEnsemble.BatchedCDKLM16(_members(n, nx, 0, bc)).batch.kernel() == (PAIR, rows)
