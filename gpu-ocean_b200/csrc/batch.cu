@@ -223,8 +223,10 @@ void batch_pick(go_batch* b) {
             // 32 rows / the height taken: periodic sides, 100 members of 195^2 276 /
             // 245, 12 of 700^2 311 / 269, 32 of 300^2 189 / 162; closed ones, whose
             // outer column blocks are frame, 12 of 700^2 312 / 303, 32 of 300^2 234 /
-            // 210, 16 of 512^2 278 / 267).  Without region strips (closed sides and
-            // at most two column blocks) the height says nothing.
+            // 210, 16 of 512^2 278 / 267).  Strips above 36 rows only where all run at
+            // once: in several waves the fit puts them too low (100 of 512^2 73 rows
+            // 1172, 32 rows 1137; 30 of 1024^2 79 rows 1215, 34 rows 1183).  Without region
+            // strips (closed sides and at most two column blocks) the height says nothing.
             b->shape = GO_SHAPE_PAIR;
             std::vector<long long> columns(n);
             for (int m = 0; m < n; ++m) {
@@ -236,7 +238,7 @@ void batch_pick(go_batch* b) {
                 long long blocks = 0;
                 for (int m = 0; m < n; ++m)
                     blocks += columns[m] * ((std::max(b->members[m]->k.ny - 4, 1) + r - 1) / r);
-                if (blocks == 0) break;
+                if (blocks == 0 || (r > 36 && blocks > 148LL * shape_blocks_per_sm(GO_SHAPE_PAIR))) continue;
                 const double cost = pair_strip_cost(blocks, r);
                 if (best < 0.0 || cost < best) { best = cost; b->rows = r; }
             }

@@ -145,7 +145,8 @@ def test_default_kernel_of_small_batches_with_land():
     assert BatchedEnsemble.BatchedCDKLM16(_members(4, 420, 1, PERIODIC)).batch.kernel() == (4, 16)
 
 
-@pytest.mark.parametrize("n,nx,bc,rows", [(12, 700, CLOSED, 29), (12, 700, PERIODIC, 22), (40, 240, CLOSED, 32)])
+@pytest.mark.parametrize("n,nx,bc,rows", [(12, 700, CLOSED, 29), (12, 700, PERIODIC, 22), (40, 240, CLOSED, 32),
+                                             (16, 512, PERIODIC, 37), (100, 260, PERIODIC, 24)])
 def test_strip_heights_of_batches_count_the_region_strips(n, nx, bc, rows):
     """Closed east and west sides: the outer column blocks are frame, and with
     two column blocks there are no others."""
