@@ -176,6 +176,8 @@ class MisfitProblem:
                                      friction_law=d.friction_law, north=(d.north_x, d.north_y))
         self.domain.set_coriolis(sim.coriolis_rows)
         self.domain.set_land(has_land)
+        if sim._domain.least_depth is not None:
+            self.domain.set_depth(sim._domain.least_depth)
         self.Hi = sim.bathymetry.Bi.tensor
         self.Hi_pitch = int(sim.bathymetry.Bi.pitch)
         self.land = float(sim.bathymetry.mask_value)
@@ -521,6 +523,8 @@ class BatchedMisfitProblem:
                                  north=(d.north_x, d.north_y))
             dom.set_coriolis(s.coriolis_rows)
             dom.set_land(_has_land(s))
+            if s._domain.least_depth is not None:
+                dom.set_depth(s._domain.least_depth)
             dom.set_wind_field(self.wind[m, 0], self.wind[m, 0], self.wind[m, 1], self.wind[m, 1])
             self.domains.append(dom)
         self.batch = _native.Batch(self.domains)

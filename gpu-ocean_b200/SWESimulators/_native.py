@@ -94,6 +94,7 @@ SIGNATURES = {
     "go_domain_set_arith": (_I, [_P, _I]),
     "go_check_quotients": (_I, [_P, _P, _P, _I, _P, _P]),
     "go_domain_set_land": (_I, [_P, _I]),
+    "go_domain_set_depth": (_I, [_P, _F]),
     "go_init_bathymetry": (_I, [_P, _P, _P, _I, _P, _I, _F]),
     "go_boundary_condition": (_I, [_P, _P, _P, _P, _P, _I]),
     "go_cdklm_swe_2D": (_I, [_P, _P, _F, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _I,
@@ -250,6 +251,7 @@ class Domain:
         self.bc = tuple(int(b) for b in bc)
         self.bc_packed = pack_bc(*self.bc)
         self.may_have_land = True
+        self.least_depth = None
 
     def close(self):
         if getattr(self, "handle", None) is not None and self.handle.value:
@@ -301,6 +303,11 @@ class Domain:
     def set_land(self, may_have_land):
         check(load().go_domain_set_land(self.handle, int(bool(may_have_land))))
         self.may_have_land = bool(may_have_land)
+
+    def set_depth(self, least_depth):
+        """Least corner depth of the water, where it is known."""
+        check(load().go_domain_set_depth(self.handle, float(least_depth)))
+        self.least_depth = float(least_depth)
 
     def status(self, clear=False):
         v = ctypes.c_uint32()

@@ -4,10 +4,13 @@
 // the reference's floating-point flags (CDKLM16.py:196-200):
 // --ftz=true --prec-div=false --prec-sqrt=false --fmad=false.
 #include <algorithm>
+#include <math.h>
+
 #include <string>
 #include <vector>
 
 #include "cfl.h"
+#include "deep.cuh"
 #include "pair_dispatch.cuh"
 #include "pair_rows.h"
 #include "trace.h"
@@ -134,12 +137,19 @@ int go_auto_shape(const go_domain* d) {
 // 768^2 30.7 / 46.3 and 23.8 / 29.5, 1024^2 48.8 / 67.1 and 44.6 / 46.4, 1280^2
 // 70.8 / 99.6 but 71.0 / 68.1.  With land (a seventh of the corners, in patches
 // of 20 cells, so that few tiles are deep): 512^2 23.7 / 33.0 and 18.4 / 23.6,
-// 640^2 34.4 / 39.3 but 26.5 / 24.6, 1024^2 68.9 / 78.1 but 63.9 / 52.5.  Land
-// that was neither told of nor ruled out counts as land.
+// 640^2 34.4 / 39.3 but 26.5 / 24.6, 1024^2 68.9 / 78.1 but 63.9 / 52.5.  The same
+// holds for water that is not deep (deep.cuh): 768^2 37.8 / 45.2 but 32.5 / 28.8,
+// 1024^2 62.1 / 64.6 but 58.7 / 46.1; 512^2 20.7 / 28.8 and 16.0 / 18.1.  So the upper
+// limit is for domains without land whose depth, where it is told, and Coriolis
+// parameter let deep water be; land that was neither told of nor ruled out
+// counts as land.
 bool go_tile_domain(const go_domain* d) {
+    if (!d->auto_launch || d->arith != GO_ARITH_RCP || go_general_north(d)) return false;
     const long long cells = (long long)d->k.nx * d->k.ny;
-    return d->auto_launch && cells < (d->land_ruled_out ? kTileCells : 350LL * 1000LL) && d->arith == GO_ARITH_RCP &&
-           !go_general_north(d);
+    if (cells < 350LL * 1000LL) return true;
+    if (cells >= kTileCells || !d->land_ruled_out) return false;
+    const DeepBounds deep = deep_bounds(d->k, d->depth_told ? d->least_depth : nanf(""), d->f_most);
+    return deep.told || (!d->depth_told && d->f_most <= deep.f);
 }
 
 // Default shape and strip height of a domain whose launch is left to the library.
@@ -188,8 +198,10 @@ StageArgs go_stage_args(const go_domain* d, float dt, int rk_step, const float* 
     a.debug = d->debug;
     a.neg_zero = -0.0f;
     a.fric = go_friction_mode(d);
-    a.deep_lo = deep_depth(a.k);
-    a.deep_hi = deep_end(a.k);
+    const DeepBounds deep = deep_bounds(a.k, d->depth_told ? d->least_depth : nanf(""), d->f_most);
+    a.deep_lo = deep.depth;
+    a.deep_eta = deep.eta;
+    a.deep_f = deep.f;
     return a;
 }
 
@@ -352,6 +364,8 @@ int go_domain_set_coriolis(go_domain* d, const float* f_rows_host, int n) {
     GO_CUDA(cudaMemcpy(d->d_frows, f_rows_host, sizeof(float) * rows, cudaMemcpyHostToDevice));
     // the copy may return before its transfer has ended
     GO_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    d->f_most = 0.0f;
+    for (int j = 0; j < rows; ++j) d->f_most = std::max(d->f_most, fabsf(f_rows_host[j]));
     return GO_OK;
 }
 
@@ -525,6 +539,13 @@ int go_cdklm_step(go_domain* d, void* stream, int n_steps, float dt, float wind_
         if (!rc && open) rc = go_boundary_condition(d, stream, eta0, hu0, hv0, pitch0);
         if (rc) return rc;
     }
+    return GO_OK;
+}
+
+int go_domain_set_depth(go_domain* d, float least_depth) {
+    if (!d) return go_fail(GO_ERR_INVALID, "null domain");
+    d->depth_told = 1;
+    d->least_depth = least_depth;
     return GO_OK;
 }
 

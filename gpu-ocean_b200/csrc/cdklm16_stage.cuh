@@ -67,7 +67,10 @@ struct StageArgs {
     float neg_zero;              // -0.0f: the addend of the packed products (column-pair kernel)
     int fric;                    // friction law kFric* (column-pair kernel; the marching kernel has it as a template)
     unsigned debug;              // GO_DEBUG_* test hooks (go_domain_set_debug), 0 in normal runs
-    float deep_lo, deep_hi;      // corner depths of deep water lie in [deep_lo, deep_hi) (deep.cuh)
+    // deep water (deep.cuh): least corner depth, largest |eta| and |f|.  The
+    // struct stays at 320 bytes: at 328 the tile kernel's next argument lost its
+    // 16-byte alignment and it ran 2 to 4% longer.
+    float deep_lo, deep_eta, deep_f;
 };
 
 // Friction law selector.

@@ -153,6 +153,7 @@ __device__ __forceinline__ bool tile_load_fixed(const StageArgs& a, const TilePl
     const Scheme& k = a.k;
     const int lane = threadIdx.x & 31, w = warp_uniform((int)threadIdx.x >> 5);
     const long long xhi = ext_hi(a), xf = ext_f(a);
+    const float hi = deep_end(k);
     bool ok = true;
     auto corner_at = [&](int r, int c) {
         const int rr = RIM ? min(t.r0 - 2 + r, k.ny + 4) : t.r0 - 2 + r;
@@ -161,7 +162,7 @@ __device__ __forceinline__ bool tile_load_fixed(const StageArgs& a, const TilePl
         return idx_ok(o, 1, xhi, a.status) ? __ldg(at_byte(a.Hi, 4u * o)) : 0.0f;
     };
     auto keep = [&](int r, int c, float h) {
-        ok = ok && h >= a.deep_lo && h < a.deep_hi;
+        ok = ok && h >= a.deep_lo && h < hi;
         const float hc = corner(h, k);
         if (r < kTileS + 5) sm.H[tile_at(r, c)].x = hc;
         if (r >= kTileS) sm.H[tile_at(r - kTileS, c)].y = hc;
@@ -180,8 +181,7 @@ __device__ __forceinline__ bool tile_load_fixed(const StageArgs& a, const TilePl
         const float2 f = make_float2(ldg1(a.f_rows, min(r, k.ny + 3), xf, a.status),
                                      ldg1(a.f_rows, min(r + kTileS, k.ny + 3), xf, a.status));
         sm.f[threadIdx.x] = f;
-        const float most = deep_coriolis(k);
-        ok = ok && fabsf(f.x) <= most && fabsf(f.y) <= most;
+        ok = ok && fabsf(f.x) <= a.deep_f && fabsf(f.y) <= a.deep_f;
     }
     return ok;
 }
@@ -266,7 +266,7 @@ __device__ __forceinline__ bool tile_cell(const StageArgs& a, const TilePlace& t
     sm.v[o] = v;
     sm.fu[o] = plane(u, fu);
     sm.fv[o] = plane(v, fv);
-    return deep_state(e.x, u.x, v.x) && deep_state(e.y, u.y, v.y);
+    return deep_state(e.x, u.x, v.x, a.deep_eta) && deep_state(e.y, u.y, v.y, a.deep_eta);
 }
 
 // Slopes of the pair at offset o along one axis: of its velocities and of the

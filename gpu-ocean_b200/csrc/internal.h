@@ -39,6 +39,8 @@ struct go_domain {
     int land_told;           // go_domain_set_land said that the bathymetry may hold land
     int tile_steps_blocks;   // most tiles of a cooperative launch of many steps (0: none)
     int land_ruled_out;      // go_domain_set_land said that the bathymetry holds no land
+    int depth_told;          // least_depth holds what go_domain_set_depth said
+    float least_depth, f_most;   // least corner depth of the water; largest |f| of the rows
 };
 
 // Records the message of a failed call (go_last_error) and returns code.

@@ -302,7 +302,8 @@ int go_sample_wind(void* stream, const float* field, int w, int h, int nx, int n
  * kernel from its size, its east and west sides, its wind kind and what
  * go_domain_set_land told: with reciprocal quotients on a north-up grid the
  * tile kernel (32 x 16 cells per block) below 350 thousand cells, or 1.15
- * million where land was ruled out; then, with one thread per column, shape 5, 6
+ * million where land was ruled out and no told depth says that the water is
+ * shallow; then, with one thread per column, shape 5, 6
  * or 4 by the columns they compute; and shape 8 from 1500^2 cells, from 1.15
  * million (1.5 million with per-cell wind) with periodic east and west sides and
  * land ruled out, and from 2300^2 (3500^2) with land and a closed side.
@@ -343,6 +344,10 @@ int go_check_quotients(void* stream, const float* a, const float* b, int n, floa
  * Common.py:1333-1337).  1 (the default) keeps every land test of the
  * reference kernel; 0 asserts there is none and skips them. */
 int go_domain_set_land(go_domain* d, int may_have_land);
+/* Least corner depth of the water (corners that are not land), where it is
+ * known.  It changes no result: the default kernel and the form of water it
+ * counts as deep are chosen with it. */
+int go_domain_set_depth(go_domain* d, float least_depth);
 
 /* Bathymetry set-up (Common.py:1319-1389): fixes the ghost corners of Hi
  * in place (periodic wrap or wall mirror, boundary_kernels.cu:121-246) and
