@@ -161,20 +161,15 @@ __device__ __forceinline__ void pflux(float2 hm, float2 um, float2 vm, float2 hp
     }
 }
 
-// x times a constant: a scalar (two scalar multiplies) or a pair (one packed).
-__device__ __forceinline__ float2 pmulc(float2 x, float c, float2) { return pscale(x, c); }
-__device__ __forceinline__ float2 pmulc(float2 x, float2 c, float2 nz) { return pmul_nz(x, c, nz); }
-
 // pflux in deep water (deep.cuh): two wet faces of an open fan, the general
-// form's arithmetic without its selections.
-template <class C>
-__device__ __forceinline__ void pflux_deep(float2 hm, float2 um, float2 vm, float2 hp, float2 up, float2 vp, C half_g,
-                                           C g, float2 nz, float2& F0, float2& F1, float2& F2) {
+// form's arithmetic without its selections.  half_g, g: the constants as pairs.
+__device__ __forceinline__ void pflux_deep(float2 hm, float2 um, float2 vm, float2 hp, float2 up, float2 vp,
+                                           float2 half_g, float2 g, float2 nz, float2& F0, float2& F1, float2& F2) {
     auto pmul = [&](float2 x, float2 y) { return pmul_nz(x, y, nz); };
     const float2 Fp0 = pmul(hp, up), Fm0 = pmul(hm, um);
-    const float2 Fp1 = padd(pmul(Fp0, up), pmul(pmulc(hp, half_g, nz), hp));
-    const float2 Fm1 = padd(pmul(Fm0, um), pmul(pmulc(hm, half_g, nz), hm));
-    const float2 gp = pmulc(hp, g, nz), gm = pmulc(hm, g, nz);
+    const float2 Fp1 = padd(pmul(Fp0, up), pmul(pmul(hp, half_g), hp));
+    const float2 Fm1 = padd(pmul(Fm0, um), pmul(pmul(hm, half_g), hm));
+    const float2 gp = pmul(hp, g), gm = pmul(hm, g);
     const float2 cp = make_float2(sqrtf(gp.x), sqrtf(gp.y)), cm = make_float2(sqrtf(gm.x), sqrtf(gm.y));
     const float2 a1 = psub(um, cm), a2 = psub(up, cp);
     const float2 b1 = padd(um, cm), b2 = padd(up, cp);
