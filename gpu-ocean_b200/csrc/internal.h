@@ -29,7 +29,8 @@ struct go_domain {
     uint64_t bc_tex[4];      // exterior solution textures: NS cur, NS next, EW cur, EW next
     float bc_t;              // their time weight
     // column-pair launches: the boundary-frame kernel runs on a second
-    // stream beside the boundary-free one (created on first use)
+    // stream beside the boundary-free one (created when land is ruled out or
+    // told of for a domain that runs it by default, else on first use)
     cudaStream_t side;
     cudaEvent_t ev_fork, ev_join;
     int own_side;            // go_domain_create's handles may create them (not the allocation-free step)
@@ -96,6 +97,7 @@ int go_launch_tile_steps(go_domain* d, cudaStream_t s, const go::StageArgs& a, i
 
 // Column-pair shape (pair_launch.cu).
 bool go_pair_shape(int shape);
+int go_pair_side(go_domain* d);     // its side stream and events, where the domain may have them (stage_launch.cu)
 namespace go { struct PairMapParams; }
 int go_prepare_pair(const go::StageArgs& a, go::PairMapParams* mp, bool* tma);
 int go_launch_pair(go_domain* d, cudaStream_t s, const go::StageArgs& a, const go::PairMapParams& mp, bool tma);

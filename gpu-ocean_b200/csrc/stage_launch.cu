@@ -30,22 +30,26 @@ Variant go_variant(const go_domain* d) {
     return v;
 }
 
+// The boundary-frame kernel's stream and the events that fork it from, and join
+// it back to, the caller's stream.
+int go_pair_side(go_domain* d) {
+    if (!d->own_side || d->side) return GO_OK;
+    int least = 0, greatest = 0;
+    GO_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    GO_CUDA(cudaStreamCreateWithPriority(&d->side, cudaStreamNonBlocking, greatest));
+    GO_CUDA(cudaEventCreateWithFlags(&d->ev_fork, cudaEventDisableTiming));
+    GO_CUDA(cudaEventCreateWithFlags(&d->ev_join, cudaEventDisableTiming));
+    return GO_OK;
+}
+
 int go_prepare_stage(go_domain* d, const StageArgs& a, PreparedStage* p) {
     p->a = a;
     p->tile = go_tile_stage(d, a);
     p->pair = !p->tile && go_pair_shape(d->shape);
     p->tma = false;
     if (!p->pair) return GO_OK;
-    if (d->own_side && !d->side) {
-        // the boundary-frame kernel's stream and the events that fork it
-        // from, and join it back to, the caller's stream
-        int least = 0, greatest = 0;
-        GO_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        GO_CUDA(cudaStreamCreateWithPriority(&d->side, cudaStreamNonBlocking, greatest));
-        GO_CUDA(cudaEventCreateWithFlags(&d->ev_fork, cudaEventDisableTiming));
-        GO_CUDA(cudaEventCreateWithFlags(&d->ev_join, cudaEventDisableTiming));
-    }
-    return go_prepare_pair(a, &p->mp, &p->tma);
+    const int rc = go_pair_side(d);
+    return rc ? rc : go_prepare_pair(a, &p->mp, &p->tma);
 }
 
 int go_launch_prepared(go_domain* d, cudaStream_t s, const PreparedStage& p, bool follows) {
