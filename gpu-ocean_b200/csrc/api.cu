@@ -36,6 +36,9 @@ int go_check_pitch(int pitch_bytes, int min_floats, const char* what) {
     return GO_OK;
 }
 
+// Least strip height: a launch's second dimension holds 65535 strips.
+static int least_rows(int ny) { return (ny + 65534) / 65535; }
+
 // Rows per block strip of the column-pair kernel, in whole ring chunks of 3
 // rows.  A strip costs its rows and about 2 more for its priming; w waves of
 // strips take the whole waves in full, and of the last, partly filled one a
@@ -49,12 +52,14 @@ int go_check_pitch(int pitch_bytes, int min_floats, const char* what) {
 // rows 177 and 134 / 24 209 and 136, 3072^2 33 rows 348 and 289 / 36 373 and 289,
 // 4096^2 30 rows 585 and 522 / 24 585 and 528, 42 611 and 517.  Strips above 36 rows
 // are left out: three simulators gain 1 to 2% with them, one alone loses as much
-// (4096^2 60 rows 597 and 513).
+// (4096^2 60 rows 597 and 513), unless the grid is so tall that the strips
+// would not fit in a launch's second dimension.
 static int pair_rows(int nx, int ny) {
     const long long strips = go::shape_columns(GO_SHAPE_PAIR, nx) / go::shape_block_width(GO_SHAPE_PAIR);
-    int best = 3;
+    const int least = (least_rows(ny) + 2) / 3 * 3;
+    int best = least;
     double best_cost = -1.0;
-    for (int r = 3; r <= 36; r += 3) {
+    for (int r = least; r <= std::max(36, least); r += 3) {
         const double cost = go::pair_strip_cost(strips * ((std::max(ny - 4, 1) + r - 1) / r), r) * (1.0 + 1.5 / r);
         if (best_cost < 0.0 || cost < best_cost) { best = r; best_cost = cost; }
     }
@@ -74,9 +79,11 @@ int go_auto_rows(int nx, int ny, int shape) {
     const long long strips = (nx + useful - 1) / useful;
     const long long slots = 148LL * go::shape_blocks_per_sm(shape);
     static const int kRows[] = {2, 4, 8, 16, 24};
-    int best = kRows[0];
+    const int least = least_rows(ny);
+    int best = std::max(kRows[0], least);
     long long best_cost = -1;
     for (int r : kRows) {
+        if (r < least) continue;
         const long long blocks = strips * ((ny + r - 1) / r);
         const long long cost = ((blocks + slots - 1) / slots) * (r + 4);
         if (best_cost < 0 || cost <= best_cost) { best = r; best_cost = cost; }

@@ -151,3 +151,14 @@ def test_strip_heights_of_batches_count_the_region_strips(n, nx, bc, rows):
     """Closed east and west sides: the outer column blocks are frame, and with
     two column blocks there are no others."""
     assert BatchedEnsemble.BatchedCDKLM16(_members(n, nx, 0, bc)).batch.kernel() == (PAIR, rows)
+
+
+@pytest.mark.parametrize("nx,ny", [(300, 2500000), (5, 2400000), (300, 60000)])
+def test_strips_of_tall_grids_fit_in_a_launch(nx, ny):
+    dom = _native.Domain(nx, ny, 1000.0, 1000.0, 9.81, bc=CLOSED)
+    for land in (False, True):
+        dom.set_land(land)
+        kernel, rows = dom.kernel()
+        assert kernel == PAIR and -(-ny // rows) <= 65535 and (rows <= 36 or ny > 36 * 65535)
+    dom.set_launch(4)
+    assert -(-ny // dom.kernel()[1]) <= 65535
