@@ -27,9 +27,9 @@
 //
 // Bounds.  Small grids wait for one tile's chain (loads, four phases) and the
 // launch; from about 600^2 cells the kernel is bound by instruction issue and
-// by the barriers of the phases: 461 instructions per cell and stage (ncu,
-// 2048^2: 176 FFMA2, 92 FADD2 and 70 FMUL per pair of cells), issue active on
-// 67% of the cycles with 32 warps per SM.  Scheme factors are kernel arguments
+// by the barriers of the phases: 469 / 486 instructions per cell in stage 0 / 1 (ncu,
+// 1024^2), with which the live rate fills 58% of the issue slots; of the warps
+// that wait, most wait at barriers.  Scheme factors are kernel arguments
 // as pairs, which a packed product takes as one operand (1002 -> 923
 // instructions per pair), and all tile arrays share one pitch, so that one
 // offset per thread addresses them (1192 -> 1002 with the interior tiles
